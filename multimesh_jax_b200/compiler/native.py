@@ -462,12 +462,15 @@ def _emit_attention_bwd(b: _Builder, ins: Instr, ids, op):
     hq = hkv * rep
     dqkv = b.new_value(ins.outs[0], qkv_r.shape, qkv_r.dtype)
     dq_acc = b.temp((B, S, hq, D), torch.float32)
-    delta = b.temp((B, hq, S), torch.float32)
-    b.call("mm_flash_attn_bwd", qkv_r, out, dout, lse, dqkv, dq_acc, delta, B, S, hkv, rep, D, STREAM)
+    rows = b.temp((b.lib.mm_flash_attn_bwd_rows(B, S, hq),), torch.float32)
+    fused = cos.shape == (S, D // 2) and cos.dtype == torch.float32
+    b.call("mm_flash_attn_bwd", qkv_r, out, dout, lse, dqkv, dq_acc, rows, cos if fused else None, sin if fused else None,
+           B, S, hkv, rep, D, STREAM)
     b.free_temp(dq_acc)
-    b.free_temp(delta)
-    n_rot = hkv * (rep + 1)
-    b.call("mm_rope", dqkv, cos, sin, B * S, cos.shape[0], n_rot, D, H * D, 1, rep + 1, rep + 2, STREAM)
+    b.free_temp(rows)
+    if not fused:
+        n_rot = hkv * (rep + 1)
+        b.call("mm_rope", dqkv, cos, sin, B * S, cos.shape[0], n_rot, D, H * D, 1, rep + 1, rep + 2, STREAM)
     b.bind(ins.outs[0], dqkv)
 
 

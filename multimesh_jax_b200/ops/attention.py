@@ -6,10 +6,9 @@ is contiguous. The softmax scale is ``1/sqrt(D)``.
 
 The packed entry points (``attention_fwd_packed`` / ``attention_bwd_packed``) run the
 tcgen05 flash-attention kernels of ``_mm_kernels.so`` (``mm_flash_attn_fwd`` /
-``mm_flash_attn_bwd``) for bf16 CUDA tensors with head dimension 128 and a sequence length
-that is a multiple of 128. Other CUDA shapes fall back to the fused scaled-dot-product
-kernels that ship with PyTorch (a library path, counted as such in the benchmarks). CPU
-tensors use an fp32 restatement.
+``mm_flash_attn_bwd``) for bf16 CUDA tensors with head dimension 128 and any sequence length.
+Other CUDA shapes fall back to the fused scaled-dot-product kernels that ship with PyTorch (a
+library path, counted as such in the benchmarks). CPU tensors use an fp32 restatement.
 """
 from __future__ import annotations
 
@@ -37,13 +36,15 @@ def have_native_kernels() -> bool:
 _lib.register("mm_flash_attn_supported", ctypes.c_int, [ctypes.c_int, ctypes.c_int])
 _lib.register("mm_flash_attn_fwd", ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
                                                   ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p])
-_lib.register("mm_flash_attn_bwd", ctypes.c_int, [ctypes.c_void_p] * 7 + [ctypes.c_int] * 5 + [ctypes.c_void_p])
+_lib.register("mm_flash_attn_bwd_rows", ctypes.c_int64, [ctypes.c_int] * 3)
+_lib.register("mm_flash_attn_bwd", ctypes.c_int, [ctypes.c_void_p] * 9 + [ctypes.c_int] * 5 + [ctypes.c_void_p])
 
 
 def native_supported(qkv: torch.Tensor) -> bool:
     """True when the packed projection can go through the tcgen05 attention kernels: CUDA,
-    bf16, contiguous, head dimension 128, sequence length a multiple of 128."""
-    if not (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.is_contiguous() and qkv.dim() == 4):
+    bf16, contiguous, 16-byte aligned, head dimension 128."""
+    if not (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.is_contiguous() and qkv.dim() == 4
+            and qkv.data_ptr() % 16 == 0):
         return False
     if os.environ.get("MM_NATIVE_ATTENTION", "1") == "0":
         return False
@@ -73,8 +74,15 @@ def attention_fwd_packed(qkv: torch.Tensor, rep: int) -> Tuple[torch.Tensor, tor
 
 
 def attention_bwd_packed(dout: torch.Tensor, qkv: torch.Tensor, out: torch.Tensor, lse: torch.Tensor,
-                         rep: int) -> torch.Tensor:
-    """Gradient of :func:`attention_fwd_packed` with respect to the packed projection."""
+                         rep: int, rope=None) -> torch.Tensor:
+    """Gradient of :func:`attention_fwd_packed` with respect to the packed projection. ``rope``: the
+    (cos, sin) tables whose rotation was applied to the query and key heads of ``qkv`` before; the
+    gradient is then the one with respect to the projection before that rotation."""
+    if rope is not None and not fuses_rope(qkv, dout, *rope):
+        B, S, H, D = qkv.shape
+        dqkv = attention_bwd_packed(dout, qkv, out, lse, rep)
+        K.rope_(dqkv.view(B * S, H, D), *rope, backward=True, rot_per_group=rep + 1, group_size=rep + 2)
+        return dqkv
     dqkv = torch.empty_like(qkv)
     if not (native_supported(qkv) and dout.dtype == torch.bfloat16):
         q, k, v = _split_packed(qkv, rep)
@@ -87,13 +95,25 @@ def attention_bwd_packed(dout: torch.Tensor, qkv: torch.Tensor, out: torch.Tenso
     dout = dout.contiguous()
     out = out.contiguous()
     dq_acc = torch.empty((B, S, hq, D), dtype=torch.float32, device=qkv.device)
-    delta = torch.empty((B, hq, S), dtype=torch.float32, device=qkv.device)
-    rc = _lib.load().mm_flash_attn_bwd(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), dqkv.data_ptr(),
-                                       dq_acc.data_ptr(), delta.data_ptr(), B, S, hkv, rep, D,
-                                       torch.cuda.current_stream().cuda_stream)
+    lib = _lib.load()
+    rows = torch.empty(lib.mm_flash_attn_bwd_rows(B, S, hq), dtype=torch.float32, device=qkv.device)
+    rc = lib.mm_flash_attn_bwd(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), dqkv.data_ptr(),
+                               dq_acc.data_ptr(), rows.data_ptr(), rope[0].data_ptr() if rope else None,
+                               rope[1].data_ptr() if rope else None, B, S, hkv, rep, D,
+                               torch.cuda.current_stream().cuda_stream)
     _lib.check(rc, "mm_flash_attn_bwd")
-    K._count(4)
+    K._count(3)
     return dqkv
+
+
+def fuses_rope(qkv: torch.Tensor, dout: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> bool:
+    """The backward kernels rotate the query and key gradients back themselves: native path, and one
+    fp32 table row per position of the sequence (a table of another length gives rows of a flattened
+    batch positions that run on across sequences, which the separate kernel handles)."""
+    S, D = qkv.shape[1], qkv.shape[3]
+    return (native_supported(qkv) and dout.dtype == torch.bfloat16 and
+            all(t.shape == (S, D // 2) and t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0
+                for t in (cos, sin)))
 
 
 def _merge_q(q):

@@ -239,10 +239,7 @@ def attention_impl(qkv, cos, sin, rep: int, inplace: bool = False):
 
 def attention_bwd_impl(dout, qkv_r, out, lse, cos, sin, rep: int):
     from .attention import attention_bwd_packed
-    B, S, H, D = qkv_r.shape
-    dqkv = attention_bwd_packed(dout, qkv_r, out, lse, rep)
-    K.rope_(dqkv.view(B * S, H, D), cos, sin, backward=True, rot_per_group=rep + 1, group_size=rep + 2)
-    return dqkv
+    return attention_bwd_packed(dout, qkv_r, out, lse, rep, rope=(cos, sin))
 
 
 def _attention_backward(ctx, gout, glse, gqkv):

@@ -65,3 +65,39 @@ def test_flash_attention_twice_in_a_row_is_deterministic_in_forward():
     a, la = attention.attention_fwd_packed(qkv, 1)
     b, lb = attention.attention_fwd_packed(qkv, 1)
     assert torch.equal(a, b) and torch.equal(la, lb)
+
+
+@pytest.mark.parametrize("B,S,hkv,rep", [(2, 1, 2, 1), (1, 17, 1, 2), (2, 63, 1, 1), (2, 65, 2, 1), (1, 127, 2, 2),
+                                         (3, 129, 1, 4), (2, 200, 2, 1), (1, 333, 2, 4), (2, 1000, 1, 1)])
+def test_flash_attention_on_ragged_sequences(B, S, hkv, rep):
+    """Sequence lengths around the tiles' edges (64 keys / queries, 128 rows): forward, log-sum-exp and
+    gradient against the fp32 restatement with the same bounds as above (P and dS rounded to bf16:
+    2^-9 per element, 1e-2 / 2e-2 of the norm), plus the gradient rotated back inside the kernels
+    against the separate rotation pass (one bf16 rounding less: 2^-8 of the norm)."""
+    from multimesh_jax_b200.ops import attention, kernels as K
+    torch.manual_seed(S + rep)
+    dev = torch.device("cuda")
+    D = 128
+    qkv = (torch.randn(B, S, hkv * (rep + 2), D, device=dev) * 0.7).bfloat16()
+    dout = torch.randn(B, S, hkv * rep, D, device=dev).bfloat16()
+    assert attention.native_supported(qkv)
+    before = K.library_call_count
+    out, lse = attention.attention_fwd_packed(qkv, rep)
+    dqkv = attention.attention_bwd_packed(dout, qkv, out, lse, rep)
+    rope = K.rope_tables(S, D, 1e4, dev)
+    assert attention.fuses_rope(qkv, dout, *rope)
+    rotated = attention.attention_bwd_packed(dout, qkv, out, lse, rep, rope=rope)
+    assert K.library_call_count == before and K.read_status() == 0
+    o_ref, lse_ref, dx_ref = _reference(qkv, rep, dout)
+    fro = lambda a, b: ((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-6)).item()
+    assert fro(out, o_ref) < 1e-2, fro(out, o_ref)
+    torch.testing.assert_close(lse, lse_ref, rtol=1e-3, atol=2e-3)
+    g, gr = dqkv.float().view(B, S, hkv, rep + 2, D), dx_ref.view(B, S, hkv, rep + 2, D)
+    if S == 1:      # a single key: the probabilities are constant and so only the value gradient is not zero
+        assert g[..., :rep + 1, :].abs().max() < 1e-2 * g[..., rep + 1, :].abs().max()
+        assert fro(g[..., rep + 1, :], gr[..., rep + 1, :]) < 1e-2
+        return
+    for slot in [slice(0, rep), rep, rep + 1]:
+        assert fro(g[:, :, :, slot], gr[:, :, :, slot]) < 2e-2, (slot, fro(g[:, :, :, slot], gr[:, :, :, slot]))
+    want = K.rope_(dqkv.clone().view(B * S, -1, D), *rope, backward=True, rot_per_group=rep + 1, group_size=rep + 2)
+    assert fro(rotated.view(B * S, -1, D), want) < 2 ** -8
