@@ -1,0 +1,83 @@
+"""The grouped mixture-of-experts kernels against a 64-bit restatement and the loop over the experts."""
+import pytest
+import torch
+
+from multimesh_jax_b200.ops import kernels as K
+from multimesh_jax_b200.ops import moe
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(x, wr, wgu, wdown, k, dy):
+    """Forward and gradients in fp64, every expert on every token."""
+    x, wr, wgu, wdown = (t.double().requires_grad_(True) for t in (x, wr, wgu, wdown))
+    topv, topi = (x @ wr.t()).topk(k, dim=-1)
+    gates = torch.softmax(topv, dim=-1)
+    y = 0
+    for e in range(wgu.shape[0]):
+        g = (gates * (topi == e)).sum(-1, keepdim=True)
+        y = y + g * ((torch.nn.functional.silu(x @ wgu[e, 0].t()) * (x @ wgu[e, 1].t())) @ wdown[e].t())
+    return [y.detach(), *torch.autograd.grad(y, (x, wr, wgu, wdown), dy.double())]
+
+
+def _inputs(T, D, F, E):
+    g = torch.Generator(device="cuda").manual_seed(T + D)
+    r = lambda *s, scale=1.0: (torch.randn(*s, device="cuda", generator=g) * scale).bfloat16()
+    return r(T, D), r(E, D, scale=D ** -0.5), r(E, 2, F, D, scale=D ** -0.5), r(E, D, F, scale=F ** -0.5), r(T, D)
+
+
+# one token; groups of a few rows; groups that end inside / on a 64- and a 256-row block; widths that are
+# no multiple of a tile or of 64; one choice, four choices, a single expert, many experts
+SIZES = [(1, 64, 64, 2, 2), (3, 128, 72, 8, 2), (300, 512, 1024, 4, 2), (257, 264, 328, 3, 1), (512, 256, 512, 1, 1),
+         (640, 128, 192, 64, 4), (1500, 1024, 1408, 8, 2)]
+
+
+@pytest.mark.parametrize("T,D,F,E,k", SIZES)
+def test_grouped_block_matches_64_bit(T, D, F, E, k):
+    x, wr, wgu, wdown, dy = _inputs(T, D, F, E)
+    assert moe._grouped_workspace(x, wr, wgu, wdown, k, True) is not None
+    before = K.library_call_count
+    got = [moe.moe_ffn_impl(x, wr, wgu, wdown, k), *moe.moe_ffn_bwd_impl(dy, x, wr, wgu, wdown, k)]
+    assert K.read_status() == 0 and K.library_call_count == before
+    for name, a, b in zip(("y", "dx", "dwr", "dwgu", "dwdown"), got, _exact(x, wr, wgu, wdown, k, dy)):
+        # at most four bf16 roundings (2^-9 each, 2^-9 / sqrt(3) in the mean square) lie on a path to an
+        # output; a gate's gradient is a difference of nearly equal sums, which doubles what reaches dwr
+        tol = 2e-2 if name == "dwr" else 1e-2
+        err = ((a.double() - b).norm() / b.norm().clamp_min(1e-30)).item()
+        assert err <= tol, (name, err)
+
+
+def test_grouped_block_with_an_expert_that_gets_nothing():
+    x, wr, wgu, wdown, dy = _inputs(200, 128, 256, 4)
+    x = x.abs()
+    wr[2] = -1.0
+    y = moe.moe_ffn_impl(x, wr, wgu, wdown, 2)
+    wgu2, wdown2 = wgu.clone(), wdown.clone()
+    wgu2[2], wdown2[2] = float("nan"), float("inf")     # must not leak into its neighbours' tiles
+    assert torch.equal(moe.moe_ffn_impl(x, wr, wgu2, wdown2, 2), y)
+    dx, dwr, dwgu, dwdown = moe.moe_ffn_bwd_impl(dy, x, wr, wgu2, wdown2, 2)
+    assert all(torch.isfinite(t).all() for t in (dx, dwr, dwgu, dwdown))
+    assert not dwgu[2].any() and not dwdown[2].any() and not dwr[2].any()
+
+
+def test_grouped_block_agrees_with_the_loop_over_experts(monkeypatch):
+    x, wr, wgu, wdown, dy = _inputs(384, 256, 384, 8)
+    x = x.view(4, 96, 256).transpose(0, 1)               # strided, three dimensions
+    dy = dy.view(96, 4, 256)
+    got = [moe.moe_ffn_impl(x, wr, wgu, wdown, 2), *moe.moe_ffn_bwd_impl(dy, x, wr, wgu, wdown, 2)]
+    monkeypatch.setattr(moe, "GROUPED_WORKSPACE_LIMIT", -1)
+    want = [moe.moe_ffn_impl(x, wr, wgu, wdown, 2), *moe.moe_ffn_bwd_impl(dy, x, wr, wgu, wdown, 2)]
+    for a, b in zip(got, want):
+        assert a.shape == b.shape and a.dtype == b.dtype
+        assert ((a.float() - b.float()).norm() / b.float().norm()).item() <= 2e-2   # both within 1e-2 of the exact result
+
+
+def test_grouped_block_keeps_a_nan_token_to_itself():
+    x, wr, wgu, wdown, dy = _inputs(130, 128, 128, 4)
+    want = moe.moe_ffn_impl(x, wr, wgu, wdown, 2)
+    x2 = x.clone()
+    x2[7, 3] = float("nan")
+    y = moe.moe_ffn_impl(x2, wr, wgu, wdown, 2)
+    assert torch.isnan(y[7]).all()
+    keep = torch.arange(130, device="cuda") != 7
+    torch.testing.assert_close(y[keep], want[keep], rtol=0, atol=0)
