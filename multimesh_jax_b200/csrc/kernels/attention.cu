@@ -42,6 +42,9 @@
 // before these changes: 5,200 cycles per 64-query step, the eight compute warps busy for 4,500
 // of them (exponentials 1,280, dS 970, the dQ reductions 1,320), the MMA lane issuing its 32
 // small (N = 64) instructions in 2,300.
+// The MMA lane's share fell when it became an elected lane with its descriptors made once (see elect_one
+// in ptx.cuh): whole call of forward + backward, B1 S8192 32 / 8 heads 3.04 -> 2.85 ms, B4 H16 S1000
+// 0.249 -> 0.233 ms.
 #include <math.h>
 
 #include "host_common.h"
@@ -102,7 +105,7 @@ __global__ void __launch_bounds__(FA_THREADS, 2)
   uint64_t* pv_done = bars + 14;    // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int q_blk = gridDim.x - 1 - blockIdx.x;  // longest rows first
   const int hq = blockIdx.y, b = blockIdx.z;
   const int g = hq / p.rep, r = hq - g * p.rep;
@@ -138,7 +141,7 @@ __global__ void __launch_bounds__(FA_THREADS, 2)
   const uint32_t tO = tmem_base + 128;  // 128-column output accumulator
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, FA_SQ);
       tma_load_4d(sQ, &tmQ, q_full, 0, hp_q, q_blk * FA_BM, b);
       tma_load_4d(sQ + FA_BM * 128, &tmQ, q_full, 64, hp_q, q_blk * FA_BM, b);
@@ -159,21 +162,20 @@ __global__ void __launch_bounds__(FA_THREADS, 2)
         for (int i = 0; i < 2000; ++i) __nanosleep(1000);  // let copies in flight land before exit
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(FA_BM, FA_BN, false, false);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(FA_BM, FA_D, false, true);
-      const uint32_t q_base = smem_u32(sQ), p_base = smem_u32(sP);
+      const uint64_t desc_q = umma_desc_sw128(smem_u32(sQ), 16, 1024), desc_k = umma_desc_sw128(smem_u32(sK), 16, 1024);
+      const uint64_t desc_p = umma_desc_sw128(smem_u32(sP), 16, 1024), desc_v = umma_desc_sw128(smem_u32(sV), FA_BN * 128, 1024);
       auto issue_s = [&](int j) {
         const int st = j & 1;
-        const uint32_t k_base = smem_u32(sK + st * FA_SKV);
+        const uint64_t dk = umma_desc_at(desc_k, st * FA_SKV);
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            const uint64_t da = umma_desc_sw128(q_base + h * (FA_BM * 128) + kk * 32, 16, 1024);
-            const uint64_t db = umma_desc_sw128(k_base + h * (FA_BN * 128) + kk * 32, 16, 1024);
-            umma_bf16(tS + st * FA_BN, da, db, idesc_s, (h | kk) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < 4; ++kk)
+            umma_bf16(tS + st * FA_BN, umma_desc_at(desc_q, h * (FA_BM * 128) + kk * 32),
+                      umma_desc_at(dk, h * (FA_BN * 128) + kk * 32), idesc_s, (h | kk) ? 1u : 0u);
         umma_commit(&s_full[st]);
         umma_commit(&k_empty[st]);
       };
@@ -193,13 +195,10 @@ __global__ void __launch_bounds__(FA_THREADS, 2)
         if (!mbar_wait(&v_full[j & 1], (j >> 1) & 1, err, MM_ERR_ATTN_WAIT) ||
             !mbar_wait(p_ready, j & 1, err, MM_ERR_ATTN_WAIT)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t v_base = smem_u32(sV + (j & 1) * FA_SKV);
+        const uint64_t dv = umma_desc_at(desc_v, (j & 1) * FA_SKV);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const uint64_t da = umma_desc_sw128(p_base + kk * 32, 16, 1024);
-          const uint64_t db = umma_desc_sw128(v_base + kk * 2048, FA_BN * 128, 1024);
-          umma_bf16(tO, da, db, idesc_pv, (j | kk) ? 1u : 0u);
-        }
+        for (int kk = 0; kk < 4; ++kk)
+          umma_bf16(tO, umma_desc_at(desc_p, kk * 32), umma_desc_at(dv, kk * 2048), idesc_pv, (j | kk) ? 1u : 0u);
         umma_commit(pv_done);
         umma_commit(&v_empty[j & 1]);
       }
@@ -384,7 +383,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dqt_free + 1);
   float* sRow = reinterpret_cast<float*>(sDST + FB_SPT + 256);   // [FB_QST][lse 64 | delta 64]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int jb = blockIdx.x;  // key block; block 0 has the most query blocks and starts first
   const int g = blockIdx.y, b = blockIdx.z;
   const int Hq = p.Hkv * p.rep;
@@ -429,7 +428,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
   const uint32_t tDK = tmem_base + 384;   // 128
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * FB_SKV);
       tma_load_4d(sK, &tmKV, kv_full, 0, hp_k, jb * FB_BKV, b);
       tma_load_4d(sK + FB_BKV * 128, &tmKV, kv_full, 64, hp_k, jb * FB_BKV, b);
@@ -458,28 +457,32 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
         for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_st = umma_idesc_bf16(FB_BKV, FB_BQ, false, false);   // K Q^T, V dO^T
       constexpr uint32_t idesc_acc = umma_idesc_bf16(FB_BKV, FA_D, false, true);    // P^T dO, dS^T Q
       constexpr uint32_t idesc_dqt = umma_idesc_bf16(FA_D, FB_BQ, true, true);      // K^T dS^T
-      const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV);
-      const uint32_t pt_base = smem_u32(sPT), dst_base = smem_u32(sDST);
-      auto issue_scores = [&](uint32_t tdst, uint32_t a_base, uint32_t b_base) {
+      // K, V, Q, dO as K-major operands of the score products; dO, Q, K, dS^T as MN-major ones of the others
+      const uint64_t desc_k = umma_desc_sw128(smem_u32(sK), 16, 1024), desc_v = umma_desc_sw128(smem_u32(sV), 16, 1024);
+      const uint64_t desc_q = umma_desc_sw128(smem_u32(sQ), 16, 1024), desc_do = umma_desc_sw128(smem_u32(sDO), 16, 1024);
+      const uint64_t desc_pt = umma_desc_sw128(smem_u32(sPT), 16, 1024), desc_dst = umma_desc_sw128(smem_u32(sDST), 16, 1024);
+      const uint64_t desc_q_mn = umma_desc_sw128(smem_u32(sQ), FB_BQ * 128, 1024);
+      const uint64_t desc_do_mn = umma_desc_sw128(smem_u32(sDO), FB_BQ * 128, 1024);
+      const uint64_t desc_k_mn = umma_desc_sw128(smem_u32(sK), FB_BKV * 128, 1024);
+      const uint64_t desc_dst_mn = umma_desc_sw128(smem_u32(sDST), FB_BKV * 128, 1024);
+      auto issue_scores = [&](uint32_t tdst, uint64_t da, uint64_t db) {
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            const uint64_t da = umma_desc_sw128(a_base + h * (FB_BKV * 128) + kk * 32, 16, 1024);
-            const uint64_t db = umma_desc_sw128(b_base + h * (FB_BQ * 128) + kk * 32, 16, 1024);
-            umma_bf16(tdst, da, db, idesc_st, (h | kk) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < 4; ++kk)
+            umma_bf16(tdst, umma_desc_at(da, h * (FB_BKV * 128) + kk * 32), umma_desc_at(db, h * (FB_BQ * 128) + kk * 32),
+                      idesc_st, (h | kk) ? 1u : 0u);
       };
       bool ok = mbar_wait(kv_full, 0, err, MM_ERR_ATTN_WAIT) && mbar_wait(&qdo_full[0], 0, err, MM_ERR_ATTN_WAIT);
       if (ok) {
         tc_fence_after();
-        issue_scores(tST, k_base, smem_u32(sQ));
+        issue_scores(tST, desc_k, desc_q);
         umma_commit(&st_full[0]);
-        issue_scores(tDPT, v_base, smem_u32(sDO));
+        issue_scores(tDPT, desc_v, desc_do);
         umma_commit(dpt_full);
       }
       for (int n = 0; n < nsteps && ok; ++n) {
@@ -489,36 +492,27 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
           if (!mbar_wait(&qdo_full[mq], (m / FB_QST) & 1, err, MM_ERR_ATTN_WAIT) ||
               !mbar_wait(&st_free[ms], ((m >> 1) & 1) ^ 1, err, MM_ERR_ATTN_WAIT)) { ok = false; break; }
           tc_fence_after();
-          issue_scores(tST + ms * FB_BQ, k_base, smem_u32(sQ + mq * FB_SQ));
+          issue_scores(tST + ms * FB_BQ, desc_k, umma_desc_at(desc_q, mq * FB_SQ));
           umma_commit(&st_full[ms]);
           if (!mbar_wait(dpt_free, n & 1, err, MM_ERR_ATTN_WAIT)) { ok = false; break; }
           tc_fence_after();
-          issue_scores(tDPT, v_base, smem_u32(sDO + mq * FB_SQ));
+          issue_scores(tDPT, desc_v, umma_desc_at(desc_do, mq * FB_SQ));
           umma_commit(dpt_full);
         }
         if (!mbar_wait(ps_ready, n & 1, err, MM_ERR_ATTN_WAIT)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t q_base = smem_u32(sQ + st * FB_SQ), do_base = smem_u32(sDO + st * FB_SQ);
+        const uint64_t dq = umma_desc_at(desc_q_mn, st * FB_SQ), ddo = umma_desc_at(desc_do_mn, st * FB_SQ);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {   // dV += P^T dO   (K = 64 query rows)
-          const uint64_t da = umma_desc_sw128(pt_base + kk * 32, 16, 1024);
-          const uint64_t db = umma_desc_sw128(do_base + kk * 2048, FB_BQ * 128, 1024);
-          umma_bf16(tDV, da, db, idesc_acc, (n | kk) ? 1u : 0u);
-        }
+        for (int kk = 0; kk < 4; ++kk)     // dV += P^T dO   (K = 64 query rows)
+          umma_bf16(tDV, umma_desc_at(desc_pt, kk * 32), umma_desc_at(ddo, kk * 2048), idesc_acc, (n | kk) ? 1u : 0u);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {   // dK += dS^T Q
-          const uint64_t da = umma_desc_sw128(dst_base + kk * 32, 16, 1024);
-          const uint64_t db = umma_desc_sw128(q_base + kk * 2048, FB_BQ * 128, 1024);
-          umma_bf16(tDK, da, db, idesc_acc, (n | kk) ? 1u : 0u);
-        }
+        for (int kk = 0; kk < 4; ++kk)     // dK += dS^T Q
+          umma_bf16(tDK, umma_desc_at(desc_dst, kk * 32), umma_desc_at(dq, kk * 2048), idesc_acc, (n | kk) ? 1u : 0u);
         if (!mbar_wait(dqt_free, (n & 1) ^ 1, err, MM_ERR_ATTN_WAIT)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {   // dQ^T = K^T dS^T   (K = 128 key rows)
-          const uint64_t da = umma_desc_sw128(k_base + kk * 2048, FB_BKV * 128, 1024);
-          const uint64_t db = umma_desc_sw128(dst_base + kk * 2048, FB_BKV * 128, 1024);
-          umma_bf16(tDQT, da, db, idesc_dqt, kk ? 1u : 0u);
-        }
+        for (int kk = 0; kk < 8; ++kk)     // dQ^T = K^T dS^T   (K = 128 key rows)
+          umma_bf16(tDQT, umma_desc_at(desc_k_mn, kk * 2048), umma_desc_at(desc_dst_mn, kk * 2048), idesc_dqt, kk ? 1u : 0u);
         umma_commit(dqt_full);
         umma_commit(&qdo_empty[st]);
       }

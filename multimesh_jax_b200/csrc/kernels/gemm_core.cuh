@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(GEMM_THREADS + 32 * Hook::kAuxWarps, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   uint8_t* epi_stage = smem + GEMM_STAGES * (GEMM_A_STAGE + GEMM_B_STAGE) + 256;  // Hook::kStageBytes
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int K = shape.depth(), N = shape.N;
   const int M = K > 0 ? shape.rows() : 0;     // nothing to contract: no tile is visited, the output is left alone
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(GEMM_THREADS + 32 * Hook::kAuxWarps, 1)
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -274,7 +274,9 @@ __global__ void __launch_bounds__(GEMM_THREADS + 32 * Hook::kAuxWarps, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
+      const uint64_t desc_a = A_MN ? umma_desc_sw128(smem_u32(sA), GEMM_BK * 128, 1024) : umma_desc_sw128(smem_u32(sA), 16, 1024);
+      const uint64_t desc_b = B_MN ? umma_desc_sw128(smem_u32(sB), GEMM_BK * 128, 1024) : umma_desc_sw128(smem_u32(sB), 16, 1024);
       constexpr uint32_t idesc = umma_idesc_bf16(GEMM_BM, GEMM_BN, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
@@ -288,16 +290,11 @@ __global__ void __launch_bounds__(GEMM_THREADS + 32 * Hook::kAuxWarps, 1)
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(&full[stage], phase, err, MM_ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t a_base = smem_u32(sA + stage * GEMM_A_STAGE);
-          const uint32_t b_base = smem_u32(sB + stage * GEMM_B_STAGE);
+          const uint64_t da = umma_desc_at(desc_a, stage * GEMM_A_STAGE), db = umma_desc_at(desc_b, stage * GEMM_B_STAGE);
 #pragma unroll
-          for (int k = 0; k < GEMM_BK / 16; ++k) {
-            const uint64_t da = A_MN ? umma_desc_sw128(a_base + k * 2048, GEMM_BK * 128, 1024)
-                                     : umma_desc_sw128(a_base + k * 32, 16, 1024);
-            const uint64_t db = B_MN ? umma_desc_sw128(b_base + k * 2048, GEMM_BK * 128, 1024)
-                                     : umma_desc_sw128(b_base + k * 32, 16, 1024);
-            umma_bf16(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < GEMM_BK / 16; ++k)
+            umma_bf16(d_tmem, umma_desc_at(da, k * (A_MN ? 2048 : 32)), umma_desc_at(db, k * (B_MN ? 2048 : 32)), idesc,
+                      (kb | k) != 0 ? 1u : 0u);
           umma_commit(&empty[stage]);
           if (++stage == GEMM_STAGES) { stage = 0; phase ^= 1; }
         }

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   int* plan = reinterpret_cast<int*>(smem + G2_STAGES * G2_STAGE_BYTES + 256);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
   int m_blk, n_blk, kb0, nkb;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -163,7 +163,9 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
+      const uint64_t desc_a = A_MN ? umma_desc_sw128(smem_u32(sA), G2_BK * 128, 1024) : umma_desc_sw128(smem_u32(sA), 16, 1024);
+      const uint64_t desc_b = (B_MN || WGRAD) ? umma_desc_sw128(smem_u32(sB), G2_BK * 128, 1024) : umma_desc_sw128(smem_u32(sB), 16, 1024);
       constexpr uint32_t idesc = umma_idesc_bf16(2 * G2_BM, G2_BN, A_MN, B_MN || WGRAD);
       int stage = 0;
       uint32_t phase = 0;
@@ -179,16 +181,11 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
         for (int i = 0; i < nkb; ++i) {
           if (!mbar_wait(&full[stage], phase, err, MM_ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t a_base = smem_u32(sA + stage * G2_A_STAGE);
-          const uint32_t b_base = smem_u32(sB + stage * G2_B_STAGE);
+          const uint64_t da = umma_desc_at(desc_a, stage * G2_A_STAGE), db = umma_desc_at(desc_b, stage * G2_B_STAGE);
 #pragma unroll
-          for (int k = 0; k < G2_BK / 16; ++k) {
-            const uint64_t da = A_MN ? umma_desc_sw128(a_base + k * 2048, G2_BK * 128, 1024)
-                                     : umma_desc_sw128(a_base + k * 32, 16, 1024);
-            const uint64_t db = (B_MN || WGRAD) ? umma_desc_sw128(b_base + k * 2048, G2_BK * 128, 1024)
-                                                : umma_desc_sw128(b_base + k * 32, 16, 1024);
-            umma_bf16_pair(d_tmem, da, db, idesc, (i | k) != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < G2_BK / 16; ++k)
+            umma_bf16_pair(d_tmem, umma_desc_at(da, k * (A_MN ? 2048 : 32)), umma_desc_at(db, k * ((B_MN || WGRAD) ? 2048 : 32)), idesc,
+                           (i | k) != 0 ? 1u : 0u);
           umma_commit_pair(&empty[stage], 3);   // frees the stage in both CTAs
           if (++stage == G2_STAGES) { stage = 0; phase ^= 1; }
         }

@@ -70,6 +70,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One lane of a fully active warp. The branches that issue TMA, tcgen05.mma and tcgen05.commit are
+// taken under this predicate and a warp-uniform warp index (below), because only then does the compiler
+// know that a single thread executes them: under `lane == 0` it guards every such instruction for a
+// divergent warp, and four MMAs with their commit took 380 cycles to issue instead of 80 - more than the
+// tensor cores need for them.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
@@ -77,6 +82,9 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(pred));
   return pred != 0;
 }
+
+// Index of this thread's warp in its block, known to be the same in every lane.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x) >> 5, 0); }
 
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -260,6 +268,9 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr, uint32_t
   d |= static_cast<uint64_t>(2) << 61;                          // SWIZZLE_128B
   return d;
 }
+// The descriptor of the same tile `bytes` further on in shared memory (a multiple of 16; the address
+// field holds all of an SM's shared memory, so the addition never carries out of it).
+__device__ __forceinline__ uint64_t umma_desc_at(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
 // Instruction descriptor for kind::f16 with bf16 inputs and fp32 accumulation.
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n, bool a_mn, bool b_mn) {
   return (1u << 4)                          // D format: F32
