@@ -16,14 +16,14 @@ static int launch_plain(const CUtensorMap& tmA, const CUtensorMap& tmB, void* C,
   cudaGetDevice(&dev);
   if (!configured[dev]) {
     MM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     GEMM_SMEM_BYTES));
+                                     GEMM_SMEM_BYTES + Hook::kStageBytes));
     configured[dev] = true;
   }
   const int num_tiles = ((M + GEMM_BM - 1) / GEMM_BM) * ((N + GEMM_BN - 1) / GEMM_BN);
   const int grid = num_tiles < ds->sm_count ? num_tiles : ds->sm_count;
   Hook hook{C, ldc, vec_ok};
   GemmShape shape{M, N, K};
-  kern<<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, stream>>>(tmA, tmB, shape, hook, ds->status);
+  kern<<<grid, GEMM_THREADS, GEMM_SMEM_BYTES + Hook::kStageBytes, stream>>>(tmA, tmB, shape, hook, ds->status);
   MM_CUDA_TRY(cudaGetLastError());
   return 0;
 }

@@ -130,6 +130,74 @@ __device__ __forceinline__ void gemm_store_chunk(void* C, int64_t ldc, int row, 
   }
 }
 
+// Drains the 32 rows of one epilogue warp (TMEM lanes of `t_base`) to rows [row0, row0 + 32) of C,
+// columns [col0, col0 + ncol), through 4 KB of shared memory: a lane holds one row of the accumulator,
+// and storing that directly touches 32 rows with 16 bytes each. Staged, a warp stores 128 contiguous
+// bytes of four rows per instruction, and accumulating reads the old values the same way, one step
+// ahead. On CTA pairs, cold operands: 1500 x 3072 x 1024 bf16 17.1 -> 12.6 us, 2048 x 2048 x 4096 fp32
+// 33.4 -> 28.2 us, 768 x 256 x 256 accumulating into fp32 17.3 -> 10.6 us.
+// Only rows below `row_limit` are written. C, its rows and `ncol` columns must be multiples of 16 bytes.
+constexpr int EPI_WARP_BYTES = 32 * 128;
+template <int OUT>
+__device__ __forceinline__ void gemm_drain_warp(uint32_t t_base, void* C, int64_t ldc, int row0, int row_limit, int col0,
+                                                int ncol, uint8_t* stage, int lane) {
+  static_assert(OUT != OUT_BF16_ACC, "accumulating into bf16 uses gemm_store_chunk");
+  constexpr bool kHalf = OUT == OUT_BF16;
+  constexpr bool kAcc = OUT == OUT_F32_ACC;
+  constexpr int CH = kHalf ? 64 : 32;       // columns per step: 128 bytes of a row
+  constexpr int esz = kHalf ? 2 : 4;
+  const int sub = lane >> 3, part = lane & 7;
+  uint8_t* base = reinterpret_cast<uint8_t*>(C) + (static_cast<int64_t>(row0) * ldc + col0) * esz + part * 16;
+  const int64_t pitch = ldc * esz;
+  const int bytes = ncol * esz - part * 16;   // of a row, from this lane's 16 bytes on
+  uint4 old[8];
+  auto fetch = [&](int c) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = i * 4 + sub;
+      old[i] = make_uint4(0, 0, 0, 0);
+      if (row0 + r < row_limit && c * esz < bytes) old[i] = *reinterpret_cast<const uint4*>(base + r * pitch + c * esz);
+    }
+  };
+  if (kAcc) fetch(0);
+#pragma unroll 1
+  for (int c = 0; c < ncol; c += CH) {
+    uint32_t lo[32], hi[32];
+    tmem_ld_32x32(t_base + c, lo);
+    if constexpr (kHalf) tmem_ld_32x32(t_base + c + 32, hi);
+    tmem_ld_wait();
+    __syncwarp();                            // the previous step's reads of the staging rows are done
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      uint4 o;
+      if constexpr (kHalf) {
+        const uint32_t(&v)[32] = i < 4 ? lo : hi;
+        const int k = (i & 3) * 8;
+        o = make_uint4(pack_bf16(__uint_as_float(v[k]), __uint_as_float(v[k + 1])),
+                       pack_bf16(__uint_as_float(v[k + 2]), __uint_as_float(v[k + 3])),
+                       pack_bf16(__uint_as_float(v[k + 4]), __uint_as_float(v[k + 5])),
+                       pack_bf16(__uint_as_float(v[k + 6]), __uint_as_float(v[k + 7])));
+      } else {
+        o = make_uint4(lo[i * 4], lo[i * 4 + 1], lo[i * 4 + 2], lo[i * 4 + 3]);
+      }
+      *reinterpret_cast<uint4*>(stage + lane * 128 + ((i ^ (lane & 7)) * 16)) = o;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = i * 4 + sub;
+      uint4 o = *reinterpret_cast<const uint4*>(stage + r * 128 + ((part ^ (r & 7)) * 16));
+      if (OUT == OUT_F32_ACC)
+        o = make_uint4(__float_as_uint(__uint_as_float(o.x) + __uint_as_float(old[i].x)),
+                       __float_as_uint(__uint_as_float(o.y) + __uint_as_float(old[i].y)),
+                       __float_as_uint(__uint_as_float(o.z) + __uint_as_float(old[i].z)),
+                       __float_as_uint(__uint_as_float(o.w) + __uint_as_float(old[i].w)));
+      if (row0 + r < row_limit && c * esz < bytes) *reinterpret_cast<uint4*>(base + r * pitch + c * esz) = o;
+    }
+    if (kAcc && c + CH < ncol) fetch(c + CH);
+  }
+}
+
 // How an epilogue warp hands a drained accumulator back to the MMA lane: an arrival on the
 // accumulator-empty barrier of its own CTA, or - in a CTA pair - of the pair's leader.
 struct TmemRelease {
@@ -158,7 +226,7 @@ struct PlainHook {
   __device__ __forceinline__ const CUtensorMap* a_map(int, const CUtensorMap* dflt) const { return dflt; }
   // Drains one 128x256 accumulator: warp `q` owns TMEM lanes [32q, 32q+32), i.e. rows
   // m_blk*128 + 32q + lane. `t_base` already points at that lane quarter.
-  static constexpr int kStageBytes = 0;  // no shared-memory staging in the epilogue
+  static constexpr int kStageBytes = 4 * EPI_WARP_BYTES;
   static constexpr int kAuxWarps = 0;    // no helper warps besides producer, MMA and epilogue
   // Row block of A / C that the scheduler's m index stands for (hooks may permute the order).
   __device__ __forceinline__ int map_m(int m_blk) const { return m_blk; }
@@ -167,16 +235,22 @@ struct PlainHook {
   __device__ __forceinline__ void finish(State&, uint8_t*, int, int, int, int, int*) const {}
   __device__ __forceinline__ void epilogue(uint32_t t_base, int m_blk, int n_blk, int q, int lane, int M, int N,
                                            int* err, uint8_t* stage, State& st, const TmemRelease& rel) const {
-    (void)err; (void)stage; (void)st;
-    const int row = m_blk * GEMM_BM + q * 32 + lane;
+    (void)err; (void)st;
+    const int row0 = m_blk * GEMM_BM + q * 32;
+    const int ncol = min(GEMM_BN, N - n_blk * GEMM_BN);
+    bool staged = false;
+    if constexpr (OUT != OUT_BF16_ACC) {
+      staged = vec_ok && ncol % (OUT == OUT_BF16 ? 8 : 4) == 0;
+      if (staged) gemm_drain_warp<OUT>(t_base, C, ldc, row0, M, n_blk * GEMM_BN, ncol, stage + q * EPI_WARP_BYTES, lane);
+    }
+    if (!staged) {
 #pragma unroll 1
-    for (int c = 0; c < GEMM_BN / 32; ++c) {
-      const int col0 = n_blk * GEMM_BN + c * 32;
-      if (col0 >= N) break;
-      uint32_t r[32];
-      tmem_ld_32x32(t_base + c * 32, r);
-      tmem_ld_wait();
-      if (row < M) gemm_store_chunk<OUT>(C, ldc, row, col0, N, r, vec_ok);
+      for (int c = 0; c < ncol; c += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32(t_base + c, r);
+        tmem_ld_wait();
+        if (row0 + lane < M) gemm_store_chunk<OUT>(C, ldc, row0 + lane, n_blk * GEMM_BN + c, N, r, vec_ok);
+      }
     }
     tc_fence_before();
     __syncwarp();

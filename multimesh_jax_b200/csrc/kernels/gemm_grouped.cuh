@@ -24,7 +24,7 @@ constexpr int GG_COUNT = GG_MAX_E;             // [64] rows that hold data
 constexpr int GG_TILE = 2 * GG_MAX_E;          // [65] 256-row tiles of the groups before this one
 constexpr int GG_PLAN = 3 * GG_MAX_E + 1;
 constexpr int GG_PAD = 64;
-constexpr int GG_SMEM_BYTES = G2_SMEM_BYTES + GG_PLAN * 4 + 12;
+constexpr int GG_SMEM_BYTES = G2_SMEM_BYTES + 4 * EPI_WARP_BYTES + GG_PLAN * 4 + 12;
 
 struct GroupedShape {
   int E, M, N, K;        // M: wgrad only; K: rows only
@@ -85,7 +85,8 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
   uint64_t* tfull = bars + 2 * G2_STAGES;  // [2]       one set per CTA
   uint64_t* tempty = tfull + 2;            // [2]       used in the leader only
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
-  int* plan = reinterpret_cast<int*>(smem + G2_STAGES * G2_STAGE_BYTES + 256);
+  uint8_t* epi_stage = smem + G2_STAGES * G2_STAGE_BYTES + 256;
+  int* plan = reinterpret_cast<int*>(epi_stage + 4 * EPI_WARP_BYTES);
 
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
@@ -217,15 +218,15 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
       if (!mbar_wait(&tfull[acc], acc_phase, err, MM_ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
       const uint32_t t_base = tmem_base + acc * G2_BN + (static_cast<uint32_t>(q * 32) << 16);
+      if (vec_ok && ncol % 8 == 0) {
+        gemm_drain_warp<OUT_BF16>(t_base, base, ldc, local - lane, limit, n_blk * G2_BN, ncol, epi_stage + q * EPI_WARP_BYTES, lane);
+      } else {
 #pragma unroll 1
-      for (int c = 0; c < ncol; c += 64) {
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32(t_base + c, r0);
-        tmem_ld_32x32(t_base + c + 32, r1);
-        tmem_ld_wait();
-        if (local < limit) {
-          gemm_store_chunk<OUT_BF16>(base, ldc, local, n_blk * G2_BN + c, shape.N, r0, vec_ok);
-          if (c + 32 < ncol) gemm_store_chunk<OUT_BF16>(base, ldc, local, n_blk * G2_BN + c + 32, shape.N, r1, vec_ok);
+        for (int c = 0; c < ncol; c += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(t_base + c, r);
+          tmem_ld_wait();
+          if (local < limit) gemm_store_chunk<OUT_BF16>(base, ldc, local, n_blk * G2_BN + c, shape.N, r, vec_ok);
         }
       }
       tc_fence_before();
