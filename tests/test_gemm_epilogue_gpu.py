@@ -30,3 +30,25 @@ def test_store_stays_inside_the_result(M, N, dtype, accumulate, pair):
         rest = flat.clone()
         rest[shift:shift + M * pitch].view(M, pitch)[:, :N] = 3.0
         assert (rest == 3.0).all()
+
+
+def test_a_thread_that_never_touched_the_device_can_launch():
+    import threading
+    a, b = torch.randn(64, 128, device="cuda").bfloat16(), torch.randn(256, 128, device="cuda").bfloat16()
+    out, seen = torch.empty(64, 256, device="cuda", dtype=torch.bfloat16), []
+    torch.cuda.synchronize()
+
+    def work():
+        try:
+            K.gemm(a, b, out=out, pair=False)
+        except Exception as e:  # noqa: BLE001 - reported below, in the test's own thread
+            seen.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    torch.cuda.synchronize()
+    assert not seen, seen
+    # 128 products: 2^-8 of a value for its rounding to bf16
+    err = ((out.float() - a.float() @ b.float().t()).norm() / out.float().norm()).item()
+    assert err <= 2.0 ** -8
