@@ -284,9 +284,8 @@ class _Builder:
         from ..ops import kernels as K
         M, Kd = (a.shape[1], a.shape[0]) if a_mn else (a.shape[0], a.shape[1])
         N = b.shape[1] if b_mn else b.shape[0]
-        pair = K.PAIR_MIN_M > 0 and M >= K.PAIR_MIN_M
-        self.call("mm_gemm_pair_bf16" if pair else "mm_gemm_bf16", a, int(a_mn), a.shape[1], b, int(b_mn), b.shape[1],
-                  out, mode, out.shape[1], M, N, Kd, STREAM)
+        self.call("mm_gemm_auto_bf16", a, int(a_mn), a.shape[1], b, int(b_mn), b.shape[1], out, mode, out.shape[1], M, N, Kd,
+                  K.PAIR_MIN_M, STREAM)
 
 
 # ------------------------------------------------------------------------------------------------

@@ -110,7 +110,8 @@ _OUT_MODE = {(bf16, False): 0, (torch.float32, False): 1, (torch.float32, True):
 
 # CTA-pair GEMM (tcgen05 cta_group::2, 256x256 tile per pair of SMs) for problems with at least
 # this many rows: 9-11 % faster than the single-CTA kernel on 8192x4096x4096 in all three layouts.
-# 0 switches it off. Environment: MM_GEMM_PAIR_MIN_M.
+# 0 switches it off. Environment: MM_GEMM_PAIR_MIN_M. Problems with too few such tiles for the
+# chip run on smaller ones whatever this says (the estimate in mm_gemm_auto_bf16).
 PAIR_MIN_M = int(os.environ.get("MM_GEMM_PAIR_MIN_M", "256"))
 
 
@@ -122,8 +123,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 
     ``a_mn`` / ``b_mn`` say that the operand is stored transposed (``[K, M]`` /
     ``[K, N]`` in memory, i.e. contiguous along M / N). Operands must be 2-D
-    with unit stride in the last dimension. ``pair`` selects the CTA-pair kernel
-    (None: by ``PAIR_MIN_M``).
+    with unit stride in the last dimension. ``pair`` selects the CTA-pair kernel or the
+    single-CTA one (None: by size, see ``PAIR_MIN_M``).
 
     ``m_dev`` / ``k_dev``: one-element int32 device tensors with the number of rows / of
     contraction elements that actually hold data; the shapes of the operands are then upper
@@ -166,12 +167,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         _lib.check(rc, "mm_gemm_pair_dyn_bf16")
         _count()
         return out
+    args = (a.data_ptr(), int(a_mn), a.stride(0), b.data_ptr(), int(b_mn), b.stride(0), out.data_ptr(), mode, out.stride(0),
+            M, N, K)
     if pair is None:
-        pair = PAIR_MIN_M > 0 and M >= PAIR_MIN_M
-    fn = lib.mm_gemm_pair_bf16 if pair else lib.mm_gemm_bf16
-    rc = fn(a.data_ptr(), int(a_mn), a.stride(0), b.data_ptr(), int(b_mn),
-            b.stride(0), out.data_ptr(), mode, out.stride(0), M, N, K, _stream())
-    _lib.check(rc, "mm_gemm_pair_bf16" if pair else "mm_gemm_bf16")
+        _lib.check(lib.mm_gemm_auto_bf16(*args, PAIR_MIN_M, _stream()), "mm_gemm_auto_bf16")
+    else:
+        fn = lib.mm_gemm_pair_bf16 if pair else lib.mm_gemm_bf16
+        _lib.check(fn(*args, _stream()), "mm_gemm_pair_bf16" if pair else "mm_gemm_bf16")
     _count()
     return out
 

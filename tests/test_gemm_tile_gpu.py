@@ -1,0 +1,45 @@
+"""The small-tile GEMM (128 x 64 and 128 x 128 tiles, contraction split over a cluster) against the fp32 product."""
+import pytest
+import torch
+
+from multimesh_jax_b200.ops import _lib
+from multimesh_jax_b200.ops import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+# one element of K per split CTA; remainders in every dimension; a ring filled once and many times; more
+# tiles than SMs (two CTAs share one)
+SIZES = [(8, 8, 8), (128, 64, 64), (136, 72, 264), (104, 200, 1000), (256, 768, 256), (304, 520, 2048), (1160, 2056, 328)]
+
+
+@pytest.mark.parametrize("M,N,Kd", SIZES)
+@pytest.mark.parametrize("bn", [64, 128])
+@pytest.mark.parametrize("split", [1, 2, 4])
+@pytest.mark.parametrize("a_mn,b_mn,mode", [(False, False, 0), (False, True, 0), (True, True, 1), (True, True, 2), (True, False, 3)])
+def test_small_tiles(M, N, Kd, bn, split, a_mn, b_mn, mode):
+    if split > (Kd + 63) // 64:
+        pytest.skip("fewer K blocks than CTAs to split them over")
+    g = torch.Generator(device="cuda").manual_seed(M + Kd)
+    a = torch.randn((Kd, M) if a_mn else (M, Kd), device="cuda", generator=g).bfloat16()
+    b = torch.randn((Kd, N) if b_mn else (N, Kd), device="cuda", generator=g).bfloat16()
+    out = torch.full((M, N), 2.0, device="cuda", dtype=torch.float32 if mode in (1, 2) else torch.bfloat16)
+    rc = _lib.load().mm_gemm_tile_bf16(a.data_ptr(), int(a_mn), a.stride(0), b.data_ptr(), int(b_mn), b.stride(0), out.data_ptr(),
+                                       mode, out.stride(0), M, N, Kd, bn, split, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and K.read_status() == 0
+    want = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double() + (2.0 if mode >= 2 else 0.0)
+    # sums of Kd products: rounding errors of the running sum, random in sign, 2^-24 sqrt(Kd) of its size;
+    # a bf16 result (8 significant bits) adds half a unit, 2^-8 of each value at most
+    err = ((out.double() - want).norm() / want.norm()).item()
+    assert err <= 4 * Kd ** 0.5 * 2.0 ** -24 + (2.0 ** -8 if mode in (0, 3) else 0.0), err
+
+
+def test_automatic_choice_is_right_at_every_size():
+    for M in (1, 40, 129, 256, 257, 1500, 4096):
+        for N in (8, 264, 2048):
+            for Kd in (8, 520, 4096):
+                a, b = torch.randn(M, Kd, device="cuda").bfloat16(), torch.randn(N, Kd, device="cuda").bfloat16()
+                want = a.float() @ b.float().t()
+                err = ((K.gemm(a, b).float() - want).norm() / want.norm()).item()
+                assert err <= 2.0 ** -8 + 4 * Kd ** 0.5 * 2.0 ** -24, (M, N, Kd, err)
+    assert K.read_status() == 0
