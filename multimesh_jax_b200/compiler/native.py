@@ -367,10 +367,9 @@ def _emit_add_rmsnorm(b: _Builder, ins: Instr, ids, op):
     if x.numel % 8:
         raise NativeUnsupported("add of a tensor whose size is not a multiple of 8")
     xn = b.new_value(ins.outs[0], x.shape, x.dtype)
-    b.call("mm_add_bf16", x, delta, xn, x.numel, STREAM)
     y = b.new_value(ins.outs[1], x.shape, x.dtype)
     rstd = b.new_value(ins.outs[2], x.shape[:-1], torch.float32)
-    b.call("mm_rmsnorm_fwd", xn, w, y, rstd, rows, D, eps, STREAM)
+    b.call("mm_add_rmsnorm_fwd", x, delta, xn, w, y, rstd, rows, D, eps, STREAM)
     b.bind(ins.outs[0], xn)
     b.bind(ins.outs[1], y)
     b.bind(ins.outs[2], rstd)
@@ -381,15 +380,12 @@ def _norm_bwd(b: _Builder, x: Sym, w: Sym, dy: Sym, rstd: Sym, dx: Sym, add_to_d
     rows = x.numel // D
     parts = b.lib.mm_rmsnorm_bwd_parts(rows)
     part = b.temp((parts, D), torch.float32)
-    dw32 = b.temp((D,), torch.float32)
-    b.call("mm_rmsnorm_bwd", x, w, dy, rstd, dx, dw32, part, rows, D, 0, int(add_to_dx), STREAM)
-    b.free_temp(part)
     dw = b.new_value(dw_vid, (D,), w.dtype)
     if w.dtype == torch.float32:
-        b.copy(dw, dw32)
+        b.call("mm_rmsnorm_bwd", x, w, dy, rstd, dx, dw, part, rows, D, 0, int(add_to_dx), STREAM)
     else:
-        b.call("mm_f32_to_bf16", dw32, dw, D, STREAM)
-    b.free_temp(dw32)
+        b.call("mm_rmsnorm_bwd_bf16", x, w, dy, rstd, dx, dw, part, rows, D, int(add_to_dx), STREAM)
+    b.free_temp(part)
     b.bind(dw_vid, dw)
 
 

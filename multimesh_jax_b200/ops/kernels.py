@@ -231,6 +231,24 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float) -> Tuple[torch.Ten
     return y, rstd
 
 
+def add_rmsnorm_fwd(x: torch.Tensor, delta: torch.Tensor, w: torch.Tensor,
+                    eps: float) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """(x + delta, its normalised rows, rstd) in one kernel for contiguous bf16 CUDA tensors of one shape."""
+    D = x.shape[-1]
+    if not (x.is_cuda and x.dtype == delta.dtype == bf16 and x.shape == delta.shape and x.is_contiguous()
+            and delta.is_contiguous() and D % 8 == 0 and x.data_ptr() % 16 == 0 and delta.data_ptr() % 16 == 0):
+        xn = add(x, delta)
+        return (xn, *rmsnorm_fwd(xn, w, eps))
+    rows = x.numel() // D
+    xn, y = torch.empty_like(x), torch.empty_like(x)
+    rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
+    rc = _lib.load().mm_add_rmsnorm_fwd(x.data_ptr(), delta.data_ptr(), xn.data_ptr(), w.data_ptr(), y.data_ptr(),
+                                        rstd.data_ptr(), rows, D, eps, _stream())
+    _lib.check(rc, "mm_add_rmsnorm_fwd")
+    _count()
+    return xn, y, rstd
+
+
 _scratch = {}
 
 

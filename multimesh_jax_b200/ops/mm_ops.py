@@ -152,8 +152,7 @@ _define("rmsnorm_bwd(Tensor x, Tensor w, Tensor dy, Tensor rstd) -> (Tensor, Ten
 
 
 def add_rmsnorm_impl(x, delta, w, eps):
-    xn = K.add(x, delta)
-    y, rstd = K.rmsnorm_fwd(xn, w, eps)
+    xn, y, rstd = K.add_rmsnorm_fwd(x, delta, w, eps)
     return xn, y, rstd.view(x.shape[:-1])
 
 

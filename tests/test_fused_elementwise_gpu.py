@@ -1,0 +1,54 @@
+"""Fused element-wise kernels against the separate ones they replace."""
+import pytest
+import torch
+
+from multimesh_jax_b200.ops import _lib
+from multimesh_jax_b200.ops import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(*shape):
+    return torch.randn(*shape, device="cuda").bfloat16()
+
+
+# one vector per row, the edges of every block size, rows that no step of two divides
+@pytest.mark.parametrize("D", [8, 1024, 1032, 2056, 4104, 16384])
+@pytest.mark.parametrize("rows", [1, 2, 3, 1301])
+def test_add_rmsnorm_and_its_weight_gradient(D, rows):
+    torch.manual_seed(D + rows)
+    x, delta, w, dy = _rand(rows, D), _rand(rows, D), _rand(D), _rand(rows, D)
+    xn, y, rstd = K.add_rmsnorm_fwd(x, delta, w, 1e-5)
+    assert torch.equal(xn, K.add(x, delta))
+    y2, rstd2 = K.rmsnorm_fwd(xn, w, 1e-5)
+    assert torch.equal(y, y2) and torch.equal(rstd, rstd2)
+    dx, dw = K.rmsnorm_bwd(xn, w, dy, rstd)
+    lib = _lib.load()
+    part = torch.empty(lib.mm_rmsnorm_bwd_parts(rows), D, device="cuda")
+    dx2, dw2 = torch.empty_like(xn), torch.empty(D, device="cuda", dtype=torch.bfloat16)
+    rc = lib.mm_rmsnorm_bwd_bf16(xn.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(), dx2.data_ptr(), dw2.data_ptr(),
+                                 part.data_ptr(), rows, D, 0, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and torch.equal(dx, dx2) and torch.equal(dw.bfloat16(), dw2)
+
+
+@pytest.mark.parametrize("F", [8, 512, 520, 1032, 11008])
+def test_swiglu_widths(F):
+    gu, dh = _rand(37, 2 * F), _rand(37, F)
+    g, u, d = gu[:, :F].double(), gu[:, F:].double(), dh.double()
+    s = torch.sigmoid(g)
+    # one bf16 rounding (2^-8 of the value at most) of a few 32-bit operations
+    torch.testing.assert_close(K.swiglu_fwd(gu).double(), g * s * u, rtol=2.0 ** -8 + 1e-5, atol=1e-6)
+    want = torch.cat([d * u * s * (1 + g * (1 - s)), d * g * s], 1)
+    torch.testing.assert_close(K.swiglu_bwd(gu, dh).double(), want, rtol=2.0 ** -8 + 1e-4, atol=1e-5)
+
+
+@pytest.mark.parametrize("n", [4, 1024, 4 * 256 * 6 * 200 + 12])     # one vector; one block; more than one pass of the grid
+def test_adamw_walks_the_whole_buffer(n):
+    torch.manual_seed(n)
+    cpu = [torch.randn(n), torch.empty(n, dtype=torch.bfloat16), torch.randn(n), torch.rand(n), torch.randn(n)]
+    gpu = [t.cuda() for t in cpu]
+    kw = dict(lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1)
+    K.adamw_step_(*cpu, step=3, **kw)
+    K.adamw_step_(*gpu, step=torch.tensor([3], device="cuda"), **kw)
+    for a, b in zip(gpu, cpu):
+        torch.testing.assert_close(a.cpu().float(), b.float(), rtol=2.0 ** -7 if b.dtype == torch.bfloat16 else 1e-5, atol=1e-6)
