@@ -433,11 +433,11 @@ def _emit_attention(b: _Builder, ins: Instr, ids, op):
         raise NativeUnsupported("attention shape outside the tcgen05 kernels")
     if b.may_overwrite(ins, ids[0]):
         qkv_r = Sym(qkv.slot, qkv.off, qkv.shape, qkv.dtype, qkv.root)
+        n_rot = H // (rep + 2) * (rep + 1)
+        b.call("mm_rope", qkv_r, cos, sin, B * S, cos.shape[0], n_rot, D, H * D, 0, rep + 1, rep + 2, STREAM)
     else:
         qkv_r = b.new_value(ins.outs[2], qkv.shape, qkv.dtype)
-        b.copy(qkv_r, qkv)
-    n_rot = H // (rep + 2) * (rep + 1)
-    b.call("mm_rope", qkv_r, cos, sin, B * S, cos.shape[0], n_rot, D, H * D, 0, rep + 1, rep + 2, STREAM)
+        b.call("mm_rope_copy", qkv, qkv_r, cos, sin, B * S, cos.shape[0], H, D, rep + 1, rep + 2, STREAM)
     hkv = H // (rep + 2)
     out = b.new_value(ins.outs[0], (B, S, hkv * rep, D), qkv.dtype)
     lse = b.new_value(ins.outs[1], (B, hkv * rep, S), torch.float32)

@@ -298,6 +298,40 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qk, const float* __restr
   *reinterpret_cast<uint4*>(base + i + half) = make_uint4(oh[0], oh[1], oh[2], oh[3]);
 }
 
+// The same rotation from `src` into another contiguous buffer, heads that are not rotated copied: one pass
+// where a copy and the in-place kernel take two. One block per token; bound by memory (with
+// the zero gradients of unused results left out, forward + backward of B1 S8192 32 / 8 heads 2.86 -> 2.81 ms).
+__global__ void __launch_bounds__(256)
+    rope_copy_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst, const float* __restrict__ cs,
+                     const float* __restrict__ sn, int S, int H, int Dh, int rot_per_group, int group_size) {
+  const int64_t t = blockIdx.x;
+  const int half = Dh / 2, per_head = half / 8;
+  const int64_t pos = t % S;
+  for (int i = threadIdx.x; i < H * per_head; i += 256) {
+    const int h = i / per_head, c0 = (i - h * per_head) * 8;
+    const int64_t at = (t * H + h) * Dh + c0;
+    uint4 lo = *reinterpret_cast<const uint4*>(src + at), hi = *reinterpret_cast<const uint4*>(src + at + half);
+    if (h % group_size < rot_per_group) {
+      const float4* cp = reinterpret_cast<const float4*>(cs + pos * half + c0);
+      const float4* sp = reinterpret_cast<const float4*>(sn + pos * half + c0);
+      const float4 ca = __ldg(cp), cb = __ldg(cp + 1), sa = __ldg(sp), sb = __ldg(sp + 1);
+      const float c[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+      const float s[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
+      uint32_t lw[4] = {lo.x, lo.y, lo.z, lo.w}, hw[4] = {hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 a = unpack_bf16(lw[j]), b = unpack_bf16(hw[j]);
+        lw[j] = pack_bf16(a.x * c[2 * j] - b.x * s[2 * j], a.y * c[2 * j + 1] - b.y * s[2 * j + 1]);
+        hw[j] = pack_bf16(b.x * c[2 * j] + a.x * s[2 * j], b.y * c[2 * j + 1] + a.y * s[2 * j + 1]);
+      }
+      lo = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+      hi = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+    }
+    *reinterpret_cast<uint4*>(dst + at) = lo;
+    *reinterpret_cast<uint4*>(dst + at + half) = hi;
+  }
+}
+
 // ------------------------------------------------------------------- SwiGLU
 // gu is [T, 2F]: gate in columns [0,F), up in [F,2F).  h = silu(gate) * up.
 // rows_dev (may be null): device-side count of the rows that hold data; rows behind it are skipped.
@@ -687,6 +721,19 @@ int mm_rope(void* qk, const float* cos_t, const float* sin_t, int64_t T, int S, 
                                                          sin_t, T, S, H, Dh, stride_t,
                                                          backward ? -1.f : 1.f, rot_per_group,
                                                          group_size);
+  MM_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
+// dst = rotated copy of src; both [T, H, Dh] contiguous, H counting the heads that are only copied.
+int mm_rope_copy(const void* src, void* dst, const float* cos_t, const float* sin_t, int64_t T, int S, int H, int Dh,
+                 int rot_per_group, int group_size, cudaStream_t stream) {
+  if (Dh % 16 || ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15)) return -2;
+  if (rot_per_group <= 0 || group_size <= 0) { rot_per_group = 1; group_size = 1; }
+  if (T == 0 || H == 0) return 0;
+  rope_copy_kernel<<<static_cast<unsigned>(T), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(src),
+                                                                 static_cast<__nv_bfloat16*>(dst), cos_t, sin_t, S, H, Dh,
+                                                                 rot_per_group, group_size);
   MM_CUDA_TRY(cudaGetLastError());
   return 0;
 }

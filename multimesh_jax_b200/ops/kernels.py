@@ -338,6 +338,20 @@ def rope_(qk: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, backward: bool
     return qk
 
 
+def rope(qk: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, rot_per_group: int = 1, group_size: int = 1) -> torch.Tensor:
+    """The rotation of :func:`rope_` into a new tensor; contiguous 16-byte aligned CUDA tensors take one kernel."""
+    T, H, Dh = qk.shape
+    if not (qk.is_cuda and qk.dtype == bf16 and qk.is_contiguous() and Dh % 16 == 0 and qk.data_ptr() % 16 == 0):
+        return rope_(qk.clone(), cos, sin, rot_per_group=rot_per_group, group_size=group_size)
+    assert H % group_size == 0
+    out = torch.empty_like(qk)
+    rc = _lib.load().mm_rope_copy(qk.data_ptr(), out.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, cos.shape[0], H, Dh,
+                                  rot_per_group, group_size, _stream())
+    _lib.check(rc, "mm_rope_copy")
+    _count()
+    return out
+
+
 # ------------------------------------------------------------------- SwiGLU
 def swiglu_fwd(gu: torch.Tensor, rows: Optional[torch.Tensor] = None) -> torch.Tensor:
     """h = silu(gate) * up. ``rows`` (one int32 on the device): only that many leading rows hold

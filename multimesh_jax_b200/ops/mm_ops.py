@@ -230,8 +230,11 @@ def attention_impl(qkv, cos, sin, rep: int, inplace: bool = False):
     derived from the tensor, so a head-sharded (tensor-parallel) slice works unchanged."""
     from .attention import attention_fwd_packed
     B, S, H, D = qkv.shape
-    qkv_r = qkv if inplace else qkv.clone()
-    K.rope_(qkv_r.view(B * S, H, D), cos, sin, rot_per_group=rep + 1, group_size=rep + 2)
+    if inplace:
+        qkv_r = qkv
+        K.rope_(qkv_r.view(B * S, H, D), cos, sin, rot_per_group=rep + 1, group_size=rep + 2)
+    else:
+        qkv_r = K.rope(qkv.contiguous().view(B * S, H, D), cos, sin, rot_per_group=rep + 1, group_size=rep + 2).view(qkv.shape)
     out, lse = attention_fwd_packed(qkv_r, rep)
     return out, lse, qkv_r
 
@@ -243,6 +246,8 @@ def attention_bwd_impl(dout, qkv_r, out, lse, cos, sin, rep: int):
 
 def _attention_backward(ctx, gout, glse, gqkv):
     qkv_r, out, lse, cos, sin = ctx.saved_tensors
+    if gout is None:
+        gout = torch.zeros_like(out)
     dqkv = torch.ops.mm_ops.attention_bwd(gout, qkv_r, out, lse, cos, sin, ctx.rep)
     return dqkv, None, None, None
 
@@ -250,6 +255,7 @@ def _attention_backward(ctx, gout, glse, gqkv):
 def _attention_setup(ctx, inputs, output):
     qkv, cos, sin, rep = inputs
     ctx.rep = rep
+    ctx.set_materialize_grads(False)    # the other two results are saved values: no zero tensor of qkv's size for them
     ctx.save_for_backward(output[2], output[0], output[1], cos, sin)
 
 

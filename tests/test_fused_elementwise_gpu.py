@@ -31,6 +31,18 @@ def test_add_rmsnorm_and_its_weight_gradient(D, rows):
     assert rc == 0 and torch.equal(dx, dx2) and torch.equal(dw.bfloat16(), dw2)
 
 
+# a table shorter and longer than the token count; one head; groups with heads that are only copied
+@pytest.mark.parametrize("T,S,H,rot,group", [(1, 1, 1, 1, 1), (300, 300, 6, 2, 3), (256, 64, 12, 5, 6), (77, 1000, 3, 2, 3)])
+def test_rotated_copy(T, S, H, rot, group):
+    x = _rand(T, H, 128)
+    cos, sin = K.rope_tables(S, 128, 1e4, "cuda")
+    out, want = K.rope(x, cos, sin, rot, group), K.rope_(x.clone(), cos, sin, rot_per_group=rot, group_size=group)
+    # the two kernels may contract products and sums differently: 2^-24 of the summands, then one bf16 rounding
+    torch.testing.assert_close(out, want, rtol=2.0 ** -7, atol=1e-5)
+    keep = torch.tensor([h % group >= rot for h in range(H)], device="cuda")
+    assert torch.equal(out[:, keep], x[:, keep])
+
+
 @pytest.mark.parametrize("F", [8, 512, 520, 1032, 11008])
 def test_swiglu_widths(F):
     gu, dh = _rand(37, 2 * F), _rand(37, F)
