@@ -590,7 +590,10 @@ def _emit_mul(b: _Builder, ins: Instr, ids, op):
     x, s = b.sym_of(ids[0]), b.sym_of(ids[1])
     if s.numel != 1 or x.dtype != torch.bfloat16 or s.dtype != torch.bfloat16:
         raise NativeUnsupported("general element-wise product")
-    out = b.new_value(ins.outs[0], x.shape, x.dtype)
+    if b.may_overwrite(ins, ids[0]):
+        out = Sym(x.slot, x.off, x.shape, x.dtype, x.root)
+    else:
+        out = b.new_value(ins.outs[0], x.shape, x.dtype)
     b.call("mm_scale_bf16", x, s, out, x.numel, STREAM)
     b.bind(ins.outs[0], out)
 
@@ -648,7 +651,40 @@ _MAY_WRITE_OVER = {
     "mm_ops.add_rmsnorm_bwd.default": ((2, 0),),
     "mm_ops.cross_entropy.default": ((0, 1),),
     "mm_ops.adamw.default": ((0, 0), (1, 1), (2, 2), (3, 3)),
+    "aten.mul.Tensor": ((0, 0),),
 }
+
+
+# operators that read their operands and write nothing but results of their own (the views among the
+# emitters hand their operand on; those that may overwrite one are named above and in INPLACE_OPERANDS)
+_VIEWS = (_emit_view, _emit_alias)
+
+
+def inputs_left_alone(cap, prog: TemplateProgram) -> set:
+    """The inputs of ``prog`` whose storage the task only reads: no operator may write over them, and
+    neither they nor a view of them is among the task's outputs. An operator this module does not
+    know counts as one that might do either."""
+    from ..ops.mm_ops import INPLACE_OPERANDS
+    source: Dict[int, int] = {v: v for v in prog.inputs}      # value -> the input whose storage it names
+    touched = set()
+    for ins in prog.instrs:
+        if ins.kind in (1, 3) and isinstance(ins.args, int):
+            if ins.args in source:
+                source[ins.outs[0]] = source[ins.args]
+            continue
+        ids = _tensor_ids_in_order(ins.args, ins.kwargs) if ins.kind != 2 else []
+        op = cap.graph.node(ins.node_id)["op"] if ins.kind in (0, 6) else None
+        emit = EMITTERS.get(op)
+        if emit in _VIEWS:
+            if ids and ids[0] in source:
+                source[ins.outs[0]] = source[ids[0]]
+        elif emit is not None:
+            written = set(INPLACE_OPERANDS.get(op, ())) | {operand for operand, _ in _MAY_WRITE_OVER.get(op, ())}
+            touched |= {source[ids[k]] for k in written if k < len(ids) and ids[k] in source}
+        elif ins.kind != 2:
+            touched |= {source[v] for v in _reads_of(ins) + ids if v in source}
+    touched |= {source[v] for v in prog.outputs if v in source}
+    return set(prog.inputs) - touched
 
 
 def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumulate: Sequence[int], have_acc: bool,

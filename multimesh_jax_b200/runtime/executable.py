@@ -13,6 +13,7 @@ from __future__ import annotations
 
 from typing import Any, Dict, List, Optional, Tuple
 
+import os
 import threading
 
 import torch
@@ -252,6 +253,7 @@ class Executable:
             if sid not in unsafe and st["kind"] == "TEMP" and st["alias_of"] < 0:
                 self._dying_inputs.setdefault(k, set()).add(sid)
         self._build_native_programs()
+        self._shared_params = self._find_shared_params()
         # Debug aid for the compiler's buffer plan (MM_CHECK_LIFETIMES=1): stores that share a
         # physical buffer must never be alive at the same time. With the knob on, every tile
         # remembers which store wrote it last; a task or reshard that reads a store whose buffer
@@ -268,6 +270,32 @@ class Executable:
                 root = plan["stores"][root["alias_of"]]
             self._alias_root[st["id"]] = root["id"]
         live_executables.add(self)
+
+    def _find_shared_params(self) -> set:
+        """Positions of arguments that need no private copy although they were not donated: every reader
+        is a task on the one local device's compute stream - which is the caller's - that only reads
+        them (:func:`inputs_left_alone`), so the step can work on the caller's own memory."""
+        from ..compiler.native import inputs_left_alone
+        plan, topo = self.plan, self.topology
+        if not (self._cuda_ctx and self._inline) or os.environ.get("MM_CHECK_LIFETIMES", "0") == "1":
+            return set()
+        d0 = topo.local_devices[0]
+        clean: Dict[int, set] = {}
+        kept = set(plan["root_stores"])
+        for st in plan["stores"]:
+            if st["alias_of"] >= 0:
+                kept |= {st["id"], st["alias_of"]}
+        for op in plan["ops"]:
+            if op["kind"] != "task":
+                kept |= {op[key] for key in ("src_store", "dst_store") if key in op}
+                continue
+            prog = self.programs[op["template"]]
+            if op["template"] not in clean:
+                clean[op["template"]] = inputs_left_alone(self.cap, prog)
+            plain = op["device_start"] == d0 and op["num_devices"] == 1 and not op["name"].endswith("_reduce")
+            kept |= {s for s, v in zip(op["inputs"], prog.inputs) if not plain or v not in clean[op["template"]]}
+            kept |= set(op["outputs"])
+        return {i for i, sid in enumerate(plan["param_stores"]) if sid >= 0 and sid not in kept}
 
     def _took_buffer(self, sid: int, d: int, old: Optional[torch.Tensor], new: torch.Tensor) -> None:
         """Store ``sid`` has just been written on device ``d`` (lifetime checking only)."""
@@ -571,7 +599,7 @@ class Executable:
                     a = shard_tensor(a.full_tensor(), want, topo)
                 new_tiles = a.local_tiles()
             else:
-                new_tiles = shard_tensor(a, want, topo, private=i not in self.donated).local_tiles()
+                new_tiles = shard_tensor(a, want, topo, private=i not in self.donated and i not in self._shared_params).local_tiles()
             self.tiles[sid].clear()
             self.tiles[sid].update(new_tiles)
             if self._lifetimes:

@@ -64,3 +64,14 @@ def test_adamw_walks_the_whole_buffer(n):
     K.adamw_step_(*gpu, step=torch.tensor([3], device="cuda"), **kw)
     for a, b in zip(gpu, cpu):
         torch.testing.assert_close(a.cpu().float(), b.float(), rtol=2.0 ** -7 if b.dtype == torch.bfloat16 else 1e-5, atol=1e-6)
+
+
+def test_scaling_in_place_by_one_and_by_another_factor():
+    x = _rand(1003)[:1000].clone()
+    for f in (1.0, -0.5):
+        want, s = (x.float() * f).bfloat16(), torch.tensor([f], device="cuda").bfloat16()
+        y = x.clone()
+        for out in (y, torch.empty_like(x)):
+            rc = _lib.load().mm_scale_bf16((y if out is y else x).data_ptr(), s.data_ptr(), out.data_ptr(), x.numel(),
+                                           torch.cuda.current_stream().cuda_stream)
+            assert rc == 0 and torch.equal(out, want)
