@@ -15,11 +15,11 @@
 //        S^T = K Q^T, dP^T = V dO^T -> TMEM; threads (one per key row) form P^T and dS^T in
 //        shared memory; dV += P^T dO, dK += dS^T Q accumulate in TMEM over the whole loop;
 //        dQ^T = K^T dS^T is read back each step and added to an fp32 dQ buffer with
-//        coalesced atomics (red.global.add.f32).
+//        row-wise reductions (red.global.add.v4.f32).
 //
 // Warp roles (both kernels): warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, the
 // others = softmax / epilogue (TMEM lane quarter = warp % 4; four warps forward, eight - two per
-// quarter, splitting the columns - backward). The backward TMA warp also brings the step's
+// quarter, splitting the columns - and four for dQ backward). The backward TMA warp also brings the step's
 // log-sum-exp and delta rows into shared memory with the step's Q / dO tiles, two steps ahead of
 // their use: as global loads of the compute warps they queued in the load/store unit behind the
 // 32 dQ reductions every thread issues per step. All waits are bounded.
@@ -47,6 +47,9 @@
 // 0.249 -> 0.233 ms.
 // Forward: the exponentials now run before the wait for the previous product, and the maximum and the sum
 // are four chains each; the scale is part of the exponent's multiply-add (same call 2.83 -> 2.77 ms).
+// Backward: dQ leaves TMEM through four warps of their own, which turn the tile around in shared memory and
+// add 512 bytes per instruction (2.76 -> 2.70 ms, the ragged case 0.227 -> 0.206). The same warps with one
+// float per lane were slower (3.06): four warps issue 256 reductions a step later than eight do.
 #include <math.h>
 
 #include "host_common.h"
@@ -329,7 +332,7 @@ constexpr int FB_SPT = FB_BKV * 128;      // P^T or dS^T: 16 KiB
 // could only be issued when step n - 1 had released its stage (0.816 -> 0.793 ms on B4 H32 S2048).
 constexpr int FB_QST = 3;
 constexpr int FB_SROW = 2 * FB_BQ * 4;    // per stage: log-sum-exp and delta of the step's 64 query rows
-constexpr int FB_SMEM = 2 * FB_SKV + 2 * FB_QST * FB_SQ + 2 * FB_SPT + 256 + FB_QST * FB_SROW;
+constexpr int FB_SMEM = 2 * FB_SKV + 2 * FB_QST * FB_SQ + 2 * FB_SPT + 256 + FB_QST * FB_SROW + FB_BQ * FA_D * 4;
 
 // Per query row: log-sum-exp in units of log2 (+inf behind the sequence, which makes every
 // probability of such a row zero) and delta = rowsum(dO * O). Stored by blocks of 64 query rows,
@@ -338,7 +341,7 @@ constexpr int FB_ROWBLK = 2 * FB_BQ;
 
 struct FaBwdParams {
   const float* rows;   // see FB_ROWBLK
-  float* dq_acc;       // [B, S, Hq, 128] fp32, zero on entry
+  float* dq_acc;       // [B, S, Hq, 128] fp32, zero on entry, without the softmax scale
   __nv_bfloat16* dqkv; // packed [B, S, Hp, 128]
   const float* cos_t;  // [>= S, 64] rotary tables, or null: the gradient is left in rotated coordinates
   const float* sin_t;
@@ -353,7 +356,7 @@ __device__ __forceinline__ void rope_bwd_pair(uint32_t& lo, uint32_t& hi, float 
   hi = __float_as_uint(b * c - a * s);
 }
 
-constexpr int FB_THREADS = 320;   // TMA warp, MMA warp, eight compute warps
+constexpr int FB_THREADS = 448;   // TMA warp, MMA warp, eight compute warps, four warps that reduce dQ
 __global__ void __launch_bounds__(FB_THREADS, 1)
     flash_bwd_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ CUtensorMap tmQ,
                      const __grid_constant__ CUtensorMap tmDO, FaBwdParams p, int* __restrict__ err) {
@@ -381,6 +384,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
   uint64_t* dqt_free = dqt_full + 1;             // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dqt_free + 1);
   float* sRow = reinterpret_cast<float*>(sDST + FB_SPT + 256);   // [FB_QST][lse 64 | delta 64]
+  float* sDQ = sRow + FB_QST * FB_ROWBLK;                         // [64 query rows][128]
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int jb = blockIdx.x;  // key block; block 0 has the most query blocks and starts first
@@ -406,7 +410,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
     mbar_init(dpt_free, 8);
     mbar_init(ps_ready, 8);
     mbar_init(dqt_full, 1);
-    mbar_init(dqt_free, 8);
+    mbar_init(dqt_free, 4);
     fence_barrier_init();
     tma_prefetch_desc(&tmKV);
     tma_prefetch_desc(&tmQ);
@@ -516,6 +520,47 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
         umma_commit(&qdo_empty[st]);
       }
     }
+  } else if (warp >= 10) {
+    // dQ^T leaves TMEM through four warps of their own, beside the next step's exponentials: a lane holds one
+    // column d of 64 query rows, the tile is turned around in shared memory, and a warp then adds whole rows
+    // (512 bytes per instruction, a quarter of the instructions that one float per lane takes).
+    const int q = warp & 3, rw = warp - 10;
+    bool ok = true;
+    for (int n = 0; n < nsteps; ++n) {
+      const int r = n / nq, i = i0 + (n - r * nq);
+      if (!mbar_wait(dqt_full, n & 1, err, MM_ERR_ATTN_WAIT)) ok = false;
+      tc_fence_after();
+      uint32_t v[32];
+      float* col = sDQ + q * 32 + lane;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        tmem_ld_32x32(tDQT + (static_cast<uint32_t>(q * 32) << 16) + h * 32, v);
+        tmem_ld_wait();
+        if (h == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dqt_free);
+        }
+#pragma unroll
+        for (int c = 0; c < 32; ++c) col[(h * 32 + c) * FA_D] = __uint_as_float(v[c]);
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (ok) {
+        float* base = p.dq_acc + ((static_cast<int64_t>(b) * p.S + i * FB_BQ) * Hq + g * p.rep + r) * FA_D + lane * 4;
+        const int64_t pitch = static_cast<int64_t>(Hq) * FA_D;
+        const int live = p.S - i * FB_BQ;   // rows of this step inside the sequence
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const int row = rw * 16 + c;
+          const float4 t = *reinterpret_cast<const float4*>(sDQ + row * FA_D + lane * 4);
+          if (row < live)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(base + row * pitch), "f"(t.x), "f"(t.y),
+                         "f"(t.z), "f"(t.w)
+                         : "memory");
+        }
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+    }
   } else {
     // Eight compute warps: two per TMEM lane quarter, each handling 32 of the step's 64 query
     // columns, so the serial chain per step (TMEM load, exp, products, shared-memory stores,
@@ -527,25 +572,9 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
     const uint32_t lane_bits = static_cast<uint32_t>(q * 32) << 16;
     const uint32_t col_off = static_cast<uint32_t>(half * 32);
     bool ok = true;
-    uint32_t dq_regs[32];
-    int prev_hq = 0, prev_i = 0;
-    auto flush_dq = [&](int hq, int i) {
-      // lane = d: 32 consecutive floats per warp and query row -> one 128-byte reduction
-      float* base = p.dq_acc + ((static_cast<int64_t>(b) * p.S + i * FB_BQ + half * 32) * Hq + hq) * FA_D + t;
-      const int live = p.S - (i * FB_BQ + half * 32);   // rows of this warp inside the sequence
-      if (live >= 32) {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) atomicAdd(base + static_cast<int64_t>(c) * Hq * FA_D, __uint_as_float(dq_regs[c]));
-      } else {
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-          if (c < live) atomicAdd(base + static_cast<int64_t>(c) * Hq * FA_D, __uint_as_float(dq_regs[c]));
-      }
-    };
     for (int n = 0; n < nsteps; ++n) {
       const int sb = n & 1;
       const int r = n / nq, i = i0 + (n - r * nq);
-      const int hq = g * p.rep + r;
       const int qcol0 = i * FB_BQ + half * 32;   // first query row (global) of this warp's columns
       const float* lse_row = sRow + (n % FB_QST) * FB_ROWBLK + half * 32;
       const float* delta_row = lse_row + FB_BQ;
@@ -569,10 +598,13 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int c = c4 * 4 + u;
-            float e = fast_exp2(__uint_as_float(s0[c]) * p.scale_log2 - lv[u]);
-            if (diag && kvg > qcol0 + c) e = 0.f;
-            s0[c] = __float_as_uint(e);
+            s0[c] = __float_as_uint(fast_exp2(__uint_as_float(s0[c]) * p.scale_log2 - lv[u]));
           }
+        }
+        if (diag) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c)
+            if (kvg > qcol0 + c) s0[c] = 0;
         }
         // ---- dS^T
         if (ok && !mbar_wait(dpt_full, n & 1, err, MM_ERR_ATTN_WAIT)) ok = false;
@@ -592,7 +624,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
           for (int u = 0; u < 4; ++u) {
             const int c = c4 * 4 + u;
             pe[u] = __uint_as_float(s0[c]);
-            de[u] = pe[u] * (__uint_as_float(d0[c]) - dv[u]) * p.scale;
+            de[u] = pe[u] * (__uint_as_float(d0[c]) - dv[u]);   // dK and dQ are scaled where they are stored
           }
           pk[c4 * 2] = pack_bf16(pe[0], pe[1]);
           pk[c4 * 2 + 1] = pack_bf16(pe[2], pe[3]);
@@ -600,16 +632,8 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
           dsk[c4 * 2 + 1] = pack_bf16(de[2], de[3]);
         }
       }
-      // ---- dQ^T of the previous step; its completion also frees sPT / sDST
-      if (n > 0) {
-        if (ok && !mbar_wait(dqt_full, (n - 1) & 1, err, MM_ERR_ATTN_WAIT)) ok = false;
-        tc_fence_after();
-        tmem_ld_32x32(tDQT + lane_bits + col_off, dq_regs);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(dqt_free);
-      }
+      // the previous step's products have read sPT and sDST
+      if (n > 0 && ok && !mbar_wait(dqt_full, (n - 1) & 1, err, MM_ERR_ATTN_WAIT)) ok = false;
       // ---- publish this warp's 32 columns (four 16-byte units per row) of P^T and dS^T
       uint8_t* prow = sPT + t * 128;
       uint8_t* drow = sDST + t * 128;
@@ -623,16 +647,10 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(ps_ready);
-      if (n > 0 && ok) flush_dq(prev_hq, prev_i);
-      prev_hq = hq;
-      prev_i = i;
     }
-    // last dQ^T, then the dK / dV accumulators
+    // every product is complete: the dK / dV accumulators
     if (ok && !mbar_wait(dqt_full, (nsteps - 1) & 1, err, MM_ERR_ATTN_WAIT)) ok = false;
     tc_fence_after();
-    tmem_ld_32x32(tDQT + lane_bits + col_off, dq_regs);
-    tmem_ld_wait();
-    if (ok) flush_dq(prev_hq, prev_i);
     if (kvg >= p.S) ok = false;
     const int Hp = p.Hkv * (p.rep + 2);
     __nv_bfloat16* krow = p.dqkv + ((static_cast<int64_t>(b) * p.S + kvg) * Hp + hp_k) * FA_D;
@@ -647,6 +665,13 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
       tmem_ld_32x32(tsrc + lane_bits + 64 + half * 32, hi);
       tmem_ld_wait();
       if (ok) {
+        if (which == 0) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            lo[c] = __float_as_uint(__uint_as_float(lo[c]) * p.scale);
+            hi[c] = __float_as_uint(__uint_as_float(hi[c]) * p.scale);
+          }
+        }
         if (which == 0 && p.cos_t) {
           const float4* ct = reinterpret_cast<const float4*>(p.cos_t + static_cast<int64_t>(kvg) * 64 + half * 32);
           const float4* st = reinterpret_cast<const float4*>(p.sin_t + static_cast<int64_t>(kvg) * 64 + half * 32);
@@ -739,11 +764,11 @@ __global__ void flash_bwd_prep_kernel(const __nv_bfloat16* __restrict__ dout, co
   }
 }
 
-// dq_acc fp32 [B, S, Hq, 128] -> bf16 query slots of the packed gradient buffer, rotated back when
+// scale * dq_acc fp32 [B, S, Hq, 128] -> bf16 query slots of the packed gradient buffer, rotated back when
 // tables are given (a thread owns 8 columns of the lower half and the same 8 of the upper one).
 __global__ void flash_dq_store_kernel(const float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv,
                                       const float* __restrict__ cos_t, const float* __restrict__ sin_t, int64_t rows, int S,
-                                      int Hkv, int rep) {
+                                      int Hkv, int rep, float scale) {
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= rows * 8) return;
   const int64_t row = idx >> 3;   // (b, s, hq)
@@ -754,10 +779,13 @@ __global__ void flash_dq_store_kernel(const float* __restrict__ dq_acc, __nv_bfl
   const int g = hq / rep, r = hq - g * rep;
   const float4* src = reinterpret_cast<const float4*>(dq_acc + row * FA_D + part * 8);
   const float4 x0 = src[0], x1 = src[1], y0 = src[16], y1 = src[17];
-  uint32_t lo[8] = {__float_as_uint(x0.x), __float_as_uint(x0.y), __float_as_uint(x0.z), __float_as_uint(x0.w),
-                    __float_as_uint(x1.x), __float_as_uint(x1.y), __float_as_uint(x1.z), __float_as_uint(x1.w)};
-  uint32_t hi[8] = {__float_as_uint(y0.x), __float_as_uint(y0.y), __float_as_uint(y0.z), __float_as_uint(y0.w),
-                    __float_as_uint(y1.x), __float_as_uint(y1.y), __float_as_uint(y1.z), __float_as_uint(y1.w)};
+  const float xf[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, yf[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+  uint32_t lo[8], hi[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    lo[i] = __float_as_uint(xf[i] * scale);
+    hi[i] = __float_as_uint(yf[i] * scale);
+  }
   if (cos_t) {
     const int64_t pos = bs % S;
     const float4* ct = reinterpret_cast<const float4*>(cos_t + pos * 64 + part * 8);
@@ -893,7 +921,7 @@ int mm_flash_attn_bwd(const void* qkv, const void* out, const void* dout, const 
   {
     const int threads = 256;
     flash_dq_store_kernel<<<static_cast<unsigned>((nrows * 8 + threads - 1) / threads), threads, 0, stream>>>(
-        dq_acc, static_cast<__nv_bfloat16*>(dqkv), cos_t, sin_t, nrows, S, Hkv, rep);
+        dq_acc, static_cast<__nv_bfloat16*>(dqkv), cos_t, sin_t, nrows, S, Hkv, rep, p.scale);
   }
   MM_CUDA_TRY(cudaGetLastError());
   return 0;
