@@ -67,7 +67,7 @@ def attention_fwd_packed(qkv: torch.Tensor, rep: int) -> Tuple[torch.Tensor, tor
     out = torch.empty((B, S, hkv * rep, D), dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty((B, hkv * rep, S), dtype=torch.float32, device=qkv.device)
     rc = _lib.load().mm_flash_attn_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), B, S, hkv, rep, D,
-                                       torch.cuda.current_stream().cuda_stream)
+                                       K._stream())
     _lib.check(rc, "mm_flash_attn_fwd")
     K._count()
     return out, lse
@@ -100,7 +100,7 @@ def attention_bwd_packed(dout: torch.Tensor, qkv: torch.Tensor, out: torch.Tenso
     rc = lib.mm_flash_attn_bwd(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), dqkv.data_ptr(),
                                dq_acc.data_ptr(), rows.data_ptr(), rope[0].data_ptr() if rope else None,
                                rope[1].data_ptr() if rope else None, B, S, hkv, rep, D,
-                               torch.cuda.current_stream().cuda_stream)
+                               K._stream())
     _lib.check(rc, "mm_flash_attn_bwd")
     K._count(3)
     return dqkv

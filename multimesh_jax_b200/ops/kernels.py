@@ -30,7 +30,8 @@ def count_library_call(n: int = 1) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the handle without a Stream object around it: every eager operator asks for it
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _count(n: int = 1) -> None:

@@ -744,7 +744,7 @@ class Executable:
                 for t_in in ins:            # allocated on another stream: keep its memory until this one is done
                     t_in.record_stream(side)
             for s, t_in, want in zip(in_ids, ins, in_shapes):
-                if tuple(t_in.shape) != want:
+                if t_in.shape != want:
                     raise RuntimeError(f"task {name}: store {s} ({stores[s]['shape']['key']}) holds a tile of shape "
                                        f"{tuple(t_in.shape)} on device {d}, expected {want}")
             if native is not None and (op["template"], d) not in self._native_off:
@@ -795,6 +795,15 @@ class Executable:
                     root_tiles[s][d] = tiles[s][d]
 
         native = self._native.get((op["template"], any(m == 2 for m in modes)))
+        out_specs = []
+        for spec in (native.outputs if native is not None else ()):
+            if spec[0] == "block":      # (tag, chunk, dtype, shape, strides, offset in elements)
+                _, chunk, off, shape, dtype = spec
+                stride, n = [0] * len(shape), 1
+                for e in reversed(range(len(shape))):
+                    stride[e], n = n, n * max(shape[e], 1)
+                spec = ("block", chunk, dtype, tuple(shape), tuple(stride), off // dtype.itemsize)
+            out_specs.append(spec)
         scratch_base = self._scratch_base.get(d, 0)
 
         def run_native(ins):
@@ -813,15 +822,17 @@ class Executable:
             native.kernel.launch(bases, scalars, torch.cuda.current_stream().cuda_stream)
             K._count(native.num_calls)
             self.native_launches += 1
-            for pos, (spec, s) in enumerate(zip(native.outputs, out_ids)):
+            typed_blocks: Dict[Tuple[int, torch.dtype], torch.Tensor] = {}
+            for pos, (spec, s) in enumerate(zip(out_specs, out_ids)):
                 if spec[0] == "acc":
                     o = tiles[s][d]
                 elif spec[0] == "block":
-                    _, chunk, off, shape, dtype = spec
-                    n = dtype.itemsize
-                    for e in shape:
-                        n *= e
-                    o = blocks[chunk][off:off + n].view(dtype).view(shape)
+                    # one view operation per output: a slice and two views of the byte block cost three
+                    _, chunk, dtype, shape, stride, off = spec
+                    typed = typed_blocks.get((chunk, dtype))
+                    if typed is None:
+                        typed = typed_blocks[chunk, dtype] = blocks[chunk].view(dtype)
+                    o = torch.as_strided(typed, shape, stride, off)
                 elif spec[0] == "ext":
                     o = ext_tiles[spec[1]].view(spec[2])
                 elif spec[0] == "slice":
