@@ -580,16 +580,25 @@ __global__ void adamw_kernel(float* __restrict__ master, __nv_bfloat16* __restri
                              float beta2, float eps, float wd, float bc1, float bc2,
                              float grad_scale, const int64_t* __restrict__ step_dev) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n4) return;
-  if (step_dev) {  // step count lives on the device: no host synchronisation per update
-    const float t = static_cast<float>(*step_dev);
-    bc1 = 1.f - powf(beta1, t);
-    bc2 = 1.f - powf(beta2, t);
+  // Memory bound (28 bytes per element) only while the arithmetic stays short: the two powers of the bias
+  // correction are computed by one thread per block, under the loads of the others (267 -> 232 us per call,
+  // the mean of a step of two 7B layers). A few blocks per SM that walk the buffer and compute them once per
+  // thread were slower: 307 us.
+  __shared__ float bc[2];
+  float4 p = make_float4(0.f, 0.f, 0.f, 0.f), mm_ = p, vv = p, g4 = p;
+  if (i < n4) {
+    p = reinterpret_cast<float4*>(master)[i];
+    mm_ = reinterpret_cast<float4*>(m)[i];
+    vv = reinterpret_cast<float4*>(v)[i];
+    g4 = reinterpret_cast<const float4*>(grad)[i];
   }
-  float4 p = reinterpret_cast<float4*>(master)[i];
-  float4 mm_ = reinterpret_cast<float4*>(m)[i];
-  float4 vv = reinterpret_cast<float4*>(v)[i];
-  const float4 g4 = reinterpret_cast<const float4*>(grad)[i];
+  if (step_dev) {  // step count lives on the device: no host synchronisation per update
+    if (threadIdx.x < 2) bc[threadIdx.x] = 1.f - powf(threadIdx.x ? beta2 : beta1, static_cast<float>(*step_dev));
+    __syncthreads();
+    bc1 = bc[0];
+    bc2 = bc[1];
+  }
+  if (i >= n4) return;
   float pa[4] = {p.x, p.y, p.z, p.w}, ma[4] = {mm_.x, mm_.y, mm_.z, mm_.w},
         va[4] = {vv.x, vv.y, vv.z, vv.w}, ga[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
