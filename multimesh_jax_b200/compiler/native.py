@@ -380,6 +380,15 @@ def _norm_bwd(b: _Builder, x: Sym, w: Sym, dy: Sym, rstd: Sym, dx: Sym, add_to_d
     rows = x.numel // D
     parts = b.lib.mm_rmsnorm_bwd_parts(rows)
     part = b.temp((parts, D), torch.float32)
+    pos = b.sole_accumulator.get(dw_vid)
+    if pos is not None:         # the column sum goes straight into the fp32 gradient accumulator
+        acc = Sym(b.acc_slot_for(pos), 0, (D,), torch.float32) if b.have_acc else b.out_region((D,), torch.float32)
+        b.call("mm_rmsnorm_bwd_acc" if w.dtype == torch.bfloat16 else "mm_rmsnorm_bwd", x, w, dy, rstd, dx, acc, part, rows, D,
+               int(b.have_acc), int(add_to_dx), STREAM)
+        b.free_temp(part)
+        b.fresh_acc[pos] = acc
+        b.bind(dw_vid, acc)
+        return
     dw = b.new_value(dw_vid, (D,), w.dtype)
     if w.dtype == torch.float32:
         b.call("mm_rmsnorm_bwd", x, w, dy, rstd, dx, dw, part, rows, D, 0, int(add_to_dx), STREAM)
@@ -744,6 +753,21 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
                 b.reaches_output.add(alias_parent[o])
                 if o in b.reaches_ext:
                     b.reaches_ext.setdefault(alias_parent[o], b.reaches_ext[o])
+    # Weight gradients of the norms that nothing but an accumulated output reads: value -> output position
+    readers: Dict[int, int] = {}
+    for ins in prog.instrs:
+        for v in _reads_of(ins):
+            readers[v] = readers.get(v, 0) + 1
+    b.sole_accumulator = {}
+    for k, v in enumerate(prog.outputs):
+        if not accumulate[k] or k in prog.fused_acc or prog.outputs.count(v) > 1:
+            continue
+        alone = readers.get(v, 0) == 0
+        while v in alias_parent and alone:
+            v = alias_parent[v]
+            alone = readers.get(v, 0) == 1 and v not in prog.outputs
+        if alone and plan_store_dtype(plan, template, k) == "float32":
+            b.sole_accumulator[v] = k
     # operand liveness inside the program, and operands other tasks still need
     last: Dict[int, int] = {}
     for idx, ins in enumerate(prog.instrs):
@@ -814,7 +838,7 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
             b.np.outputs.append(("ext", j, sym.shape, sym.dtype))
             continue
         if mode:
-            fused = prog.fused_acc.get(k)
+            fused = prog.fused_acc.get(k) or k in b.fresh_acc
             if fused:
                 if have_acc:
                     b.np.outputs.append(("acc", k))

@@ -29,6 +29,12 @@ def test_add_rmsnorm_and_its_weight_gradient(D, rows):
     rc = lib.mm_rmsnorm_bwd_bf16(xn.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(), dx2.data_ptr(), dw2.data_ptr(),
                                  part.data_ptr(), rows, D, 0, torch.cuda.current_stream().cuda_stream)
     assert rc == 0 and torch.equal(dx, dx2) and torch.equal(dw.bfloat16(), dw2)
+    acc = torch.randn(D, device="cuda")
+    for accumulate, want in ((0, dw2.float()), (1, acc + dw2.float())):
+        rc = lib.mm_rmsnorm_bwd_acc(xn.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(), dx2.data_ptr(),
+                                    (out := acc.clone()).data_ptr(), part.data_ptr(), rows, D, accumulate, 0,
+                                    torch.cuda.current_stream().cuda_stream)
+        assert rc == 0 and torch.equal(out, want)
 
 
 # a table shorter and longer than the token count; one head; groups with heads that are only copied
