@@ -12,6 +12,7 @@ analogue of the reference compiling each unique task body once
 """
 from __future__ import annotations
 
+import functools
 import json
 from typing import Any, Callable, Dict, List, Optional, Sequence, Tuple
 
@@ -91,6 +92,10 @@ class TemplateProgram:
         self.device_start = template["device_start"]
         self._last_use = last_use
         self.fused_acc: Dict[int, bool] = {}
+        # (instruction index, operand id) of the operands that an operator may write its result over
+        self.takes_over: set = set()
+        # the inputs that some operator of the task may write over
+        self.written_inputs: set = set()
 
     def run(self, ctx, scalars: Sequence[int], inputs: Sequence[torch.Tensor],
             acc_bufs: Optional[Sequence[Optional[torch.Tensor]]] = None) -> List[torch.Tensor]:
@@ -180,8 +185,148 @@ def _local_shape(value: dict) -> List[int]:
     return list(sh["shard_size"]) if sh else list(value["shape"])
 
 
+# Operators whose result is the operand itself in another shape. Any other operator that returns a view
+# (slices, transposes, broadcasts) gives a value that a kernel must not write through.
+WHOLE_VIEWS = {"aten.view.default", "aten._unsafe_view.default", "aten.reshape.default", "aten.detach.default",
+               "aten.alias.default"}
+
+
+@functools.lru_cache(maxsize=None)
+def returns_view(op: str) -> bool:
+    """Whether the result of a captured operator may lie in the memory of its first tensor operand. An
+    operator that cannot be looked up counts as one."""
+    if op in WHOLE_VIEWS:
+        return True
+    try:
+        namespace, name, overload = op.split(".")
+        schema = getattr(getattr(getattr(torch.ops, namespace), name), overload)._schema
+    except (AttributeError, ValueError):
+        return True
+    return any(r.alias_info is not None for r in schema.returns)
+
+
+def _storage_source(op: str, operands: Sequence[int]) -> Tuple[Optional[int], bool]:
+    """The operand in whose memory the results of a node lie (None: in memory of their own), and whether
+    they are all of it in the same order."""
+    if op in ("mm.accumulate", "mm.relayout", "mm.all_reduce", "mm.spmd_reshard", "mm.dynamic_slice") or op.startswith("mm.marker"):
+        return operands[0], op != "mm.dynamic_slice"
+    if op.startswith("mm.") or not operands or not returns_view(op):
+        return None, True
+    return operands[0], op in WHOLE_VIEWS
+
+
+class StorageUse:
+    """Which values of an instruction list share memory, and when the last of them is read. ``root`` maps a
+    value to the one whose memory it lies in; values that are a strided or partial view are in ``partial``."""
+
+    def __init__(self, g, instrs: Sequence[Instr], inputs: Sequence[int], outputs: Sequence[int]):
+        self.root: Dict[int, int] = {v: v for v in inputs}
+        self.partial: set = set()
+        self.inputs = set(inputs)
+        self.instrs = instrs
+        last: Dict[int, int] = {}
+        for idx, ins in enumerate(instrs):
+            for v in _reads(ins):
+                last[v] = idx
+            src, whole = None, True
+            if ins.kind in (0, 1, 3, 4, 5, 6):
+                src, whole = _storage_source(g.node(ins.node_id)["op"], _reads(ins))
+            for o in ins.outs or ():
+                self.root[o] = o if src is None else self.root.get(src, src)
+                if src is not None and (not whole or src in self.partial):
+                    self.partial.add(o)
+        self.needed_until: Dict[int, int] = {}      # root -> last instruction that reads any value in its memory
+        kept = set(outputs)
+        for v, r in self.root.items():
+            end = len(instrs) if v in kept else last.get(v, -1)
+            self.needed_until[r] = max(self.needed_until.get(r, -1), end)
+
+    def dies_with(self, idx: int, vid: int, overwritable: set) -> bool:
+        """Nothing needs the memory of ``vid`` behind instruction ``idx``, which reads it through this one
+        operand, so the instruction may write a result over it. Memory of a task input qualifies only
+        when it is in ``overwritable``."""
+        root = self.root.get(vid, vid)
+        if vid in self.partial or self.needed_until.get(root, len(self.instrs)) > idx:
+            return False
+        if root in self.inputs and root not in overwritable:
+            return False
+        return sum(self.root.get(v, v) == root for v in _reads(self.instrs[idx])) == 1
+
+
+def overwritable_inputs(cap: Captured, plan: dict) -> Dict[int, Tuple[set, set, set]]:
+    """Per template id the inputs whose memory a launch may take over, as three sets of values:
+
+    * temporaries that this launch alone reads, in every launch of the template (a store that several
+      launches read - a loop-invariant value in a microbatch loop, a value two tasks share - is in no set);
+    * step arguments that this launch alone reads;
+    * step arguments that other tasks read too, but all of them earlier in plan order.
+
+    A store that a reshard reads, that is a result of the step, or whose memory another store shares
+    (results of one task that are views of one another, an input handed on as a result) and still
+    offers to a reader is in none of them."""
+    stores, ops = plan["stores"], plan["ops"]
+    parent = list(range(len(stores)))
+
+    def find(s: int) -> int:
+        while parent[s] != s:
+            parent[s] = parent[parent[s]]
+            s = parent[s]
+        return s
+
+    readers: Dict[int, List[int]] = {}
+    moved: set = set()
+    roots: Dict[int, Dict[int, int]] = {}
+    for k, op in enumerate(ops):
+        if op["kind"] == "reshard":
+            moved.add(op["src_store"])
+        if op["kind"] != "task":
+            continue
+        t = plan["templates"][op["template"]]
+        if t["id"] not in roots:
+            root = roots[t["id"]] = {v: v for v in t["inputs"]}
+            for nid in t["nodes"]:
+                n = cap.graph.node(nid)
+                src, _ = _storage_source(n["op"], n["inputs"])
+                for o in n["outputs"]:
+                    root[o] = o if src is None else root.get(src, src)
+        root = roots[t["id"]]
+        for s in op["inputs"]:
+            readers.setdefault(s, []).append(k)
+        holder: Dict[int, int] = dict(zip(t["inputs"], op["inputs"]))
+        for v, s in zip(t["outputs"], op["outputs"]):
+            parent[find(s)] = find(holder.setdefault(root.get(v, v), s))
+    members: Dict[int, List[int]] = {}
+    for s in range(len(stores)):
+        members.setdefault(find(s), []).append(s)
+    results = set(plan["root_stores"])
+
+    def offered(s: int) -> bool:            # somebody outside the launch at hand looks at this store
+        return s in moved or s in results or stores[s]["kind"] == "ROOT"
+
+    out: Dict[int, Tuple[set, set, set]] = {}
+    for k, op in enumerate(ops):
+        if op["kind"] != "task":
+            continue
+        sets: Tuple[set, set, set] = (set(), set(), set())
+        for v, s in zip(plan["templates"][op["template"]]["inputs"], op["inputs"]):
+            others = [m for m in members[find(s)] if m != s]
+            if offered(s) or any(offered(m) or m in readers for m in others):
+                continue
+            if stores[s]["kind"] == "PARAM":
+                if max(readers[s]) == k and readers[s].count(k) == 1:
+                    sets[2].add(v)
+                    if len(readers[s]) == 1:
+                        sets[1].add(v)
+            elif len(readers[s]) == 1:
+                sets[0].add(v)
+        seen = out.get(op["template"])
+        out[op["template"]] = sets if seen is None else tuple(a & b for a, b in zip(seen, sets))
+    return out
+
+
 def build_program(cap: Captured, plan: dict, template: dict, fast_ops: Optional[Dict[str, Callable]] = None,
-                  acc_fusable: Optional[set] = None) -> TemplateProgram:
+                  acc_fusable: Optional[set] = None, overwritable: Optional[Dict[int, tuple]] = None) -> TemplateProgram:
+    """``overwritable``: the result of :func:`overwritable_inputs` for this plan, when the caller has it."""
     g = cap.graph
     instrs: List[Instr] = []
     fast_variants: List[Tuple[Instr, Callable, str]] = []   # (instruction, plain operator, op name)
@@ -429,32 +574,36 @@ def build_program(cap: Captured, plan: dict, template: dict, fast_ops: Optional[
     for idx, ins in enumerate(instrs):
         for v in _reads(ins):
             last[v] = idx
-    # A fast variant that overwrites one of its operands is only valid when nothing reads that
-    # operand afterwards (passes may have moved a reader behind it): otherwise run the plain one.
-    if fast_variants:
-        from ..ops.mm_ops import INPLACE_OPERANDS
-        # an input that another task reads as well (the two halves of a split backward task share
-        # the incoming boundary gradient) must survive this task unchanged
-        mine = set(template["inputs"])
-        shared_inputs = {v for t in plan["templates"] if t is not template and t["name"] != template["name"]
-                         for v in t["inputs"] if v in mine}
-        index_of = {id(ins): idx for idx, ins in enumerate(instrs)}
-        for ins_obj, plain, opname in fast_variants:
-            idx = index_of.get(id(ins_obj))
-            clobbered = INPLACE_OPERANDS.get(opname)
-            if idx is None or not clobbered:
-                continue
-            ids = _tensor_ids_in_order(ins_obj.args, ins_obj.kwargs)
-            for pos in clobbered:
-                if pos < len(ids) and (last.get(ids[pos], -1) > idx or ids[pos] in keep or ids[pos] in shared_inputs):
-                    ins_obj.fn = plain
-                    break
+    # An operator may write its result over an operand when nothing needs the operand's memory afterwards:
+    # no value of this task that lies in it, no other reader of the store behind a task input. The native
+    # program asks the same set; here the operators with a variant that does so fall back to the plain
+    # form (AdamW: per operand) where the rule refuses.
+    from ..ops.mm_ops import MAY_WRITE_OVER
+    temps, sole_args, last_args = (overwritable or overwritable_inputs(cap, plan)).get(template["id"], (set(), set(), set()))
+    use = StorageUse(g, instrs, template["inputs"], template["outputs"])
+    takes_over, written_inputs = set(), set()
+    plain_of = {id(ins): plain for ins, plain, _ in fast_variants}
+    for idx, ins in enumerate(instrs):
+        opname = g.node(ins.node_id)["op"] if ins.kind == 0 else None
+        if opname not in MAY_WRITE_OVER:
+            continue
+        ids = _tensor_ids_in_order(ins.args, ins.kwargs)
+        operands = [ids[pos] for pos, _ in MAY_WRITE_OVER[opname] if pos < len(ids)]
+        update = opname == "mm_ops.adamw.default"      # the one operator that may take over step arguments
+        taken = {v for v in operands if use.dies_with(idx, v, temps | sole_args if update else temps)}
+        takes_over |= {(idx, v) for v in taken}
+        # the interpreted update also writes over arguments that earlier tasks have read
+        dead = [use.dies_with(idx, v, temps | last_args if update else temps) for v in operands]
+        written_inputs |= {use.root[v] for v, d in zip(operands, dead) if d and use.root.get(v) in use.inputs}
+        if id(ins) in plain_of and not all(dead):
+            ins.fn = functools.partial(ins.fn, overwrite=tuple(dead)) if update else plain_of[id(ins)]
     last_use: Dict[int, List[int]] = {}
     for v, idx in last.items():
         if v not in keep:
             last_use.setdefault(idx, []).append(v)
     prog = TemplateProgram(template, instrs, list(template["inputs"]), list(template["outputs"]), last_use)
     prog.fused_acc = fused_acc
+    prog.takes_over, prog.written_inputs = takes_over, written_inputs
     return prog
 
 
@@ -510,6 +659,6 @@ def _fix_sizes(arg, gshape, lshape):
 def _reads(ins: Instr) -> List[int]:
     if ins.kind == 11:      # reads the row shard (not the gathered value its operator names) and the weight
         return [ins.extra[6], ins.extra[7]]
-    if ins.kind in (0, 6, 7, 10):
+    if ins.kind in (0, 6, 7, 8, 10):
         return _tensor_ids_in_order(ins.args, ins.kwargs)
     return [ins.args]

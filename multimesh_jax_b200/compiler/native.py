@@ -17,8 +17,8 @@ instruction (``src/pjrt_client/mm_pjrt_executable.cc:549-590``, ``src/pjrt_clien
 * every intermediate gets an offset inside the per-device *scratch tile* of the runtime
   context, assigned by a liveness-based first-fit allocator, so the scratch a template needs
   is the peak of its live intermediates, not their sum;
-* operators that may overwrite a dead operand do so (the rules of ``FAST_OPS`` /
-  ``INPLACE_OPERANDS``).
+* operators that may overwrite an operand do so when nothing needs its memory any more
+  (``MAY_WRITE_OVER`` names them, :class:`~multimesh_jax_b200.compiler.lower.StorageUse` decides).
 
 Pointer arguments are recorded as ``(slot, byte offset)``; the slots of a launch are its input
 tiles, the output block, the scratch tile and the gradient accumulators it adds into. A
@@ -37,7 +37,8 @@ import torch
 from ..ops import _lib
 from ..ops import attention as _attention  # noqa: F401  (declares the attention entry points)
 from .capture import DTYPE_FROM_NAME
-from .lower import Instr, TemplateProgram, _tensor_ids_in_order, _V
+from ..ops.mm_ops import MAY_WRITE_OVER
+from .lower import Instr, StorageUse, TemplateProgram, _reads, _tensor_ids_in_order, _V
 
 ALIGN = 256
 
@@ -654,45 +655,16 @@ EMITTERS = {
 }
 
 
-# operators that may write a result over a dead operand: (tensor operand position, result position)
-_MAY_WRITE_OVER = {
-    "mm_ops.attention.default": ((0, 2),),
-    "mm_ops.add_rmsnorm_bwd.default": ((2, 0),),
-    "mm_ops.cross_entropy.default": ((0, 1),),
-    "mm_ops.adamw.default": ((0, 0), (1, 1), (2, 2), (3, 3)),
-    "aten.mul.Tensor": ((0, 0),),
-}
-
-
-# operators that read their operands and write nothing but results of their own (the views among the
-# emitters hand their operand on; those that may overwrite one are named above and in INPLACE_OPERANDS)
-_VIEWS = (_emit_view, _emit_alias)
-
-
 def inputs_left_alone(cap, prog: TemplateProgram) -> set:
     """The inputs of ``prog`` whose storage the task only reads: no operator may write over them, and
     neither they nor a view of them is among the task's outputs. An operator this module does not
     know counts as one that might do either."""
-    from ..ops.mm_ops import INPLACE_OPERANDS
-    source: Dict[int, int] = {v: v for v in prog.inputs}      # value -> the input whose storage it names
-    touched = set()
+    root = StorageUse(cap.graph, prog.instrs, prog.inputs, prog.outputs).root
+    touched = set(prog.written_inputs) | {root.get(v, v) for v in prog.outputs}
     for ins in prog.instrs:
-        if ins.kind in (1, 3) and isinstance(ins.args, int):
-            if ins.args in source:
-                source[ins.outs[0]] = source[ins.args]
-            continue
-        ids = _tensor_ids_in_order(ins.args, ins.kwargs) if ins.kind != 2 else []
         op = cap.graph.node(ins.node_id)["op"] if ins.kind in (0, 6) else None
-        emit = EMITTERS.get(op)
-        if emit in _VIEWS:
-            if ids and ids[0] in source:
-                source[ins.outs[0]] = source[ids[0]]
-        elif emit is not None:
-            written = set(INPLACE_OPERANDS.get(op, ())) | {operand for operand, _ in _MAY_WRITE_OVER.get(op, ())}
-            touched |= {source[ids[k]] for k in written if k < len(ids) and ids[k] in source}
-        elif ins.kind != 2:
-            touched |= {source[v] for v in _reads_of(ins) + ids if v in source}
-    touched |= {source[v] for v in prog.outputs if v in source}
+        if ins.kind not in (1, 2, 3) and op not in EMITTERS:
+            touched |= {root.get(v, v) for v in _reads(ins)}
     return set(prog.inputs) - touched
 
 
@@ -731,11 +703,15 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
         sh = val.get("sharding")
         shape = sh["shard_size"] if sh else val["shape"]
         b.env[v] = Sym(i, 0, shape, DTYPE_FROM_NAME[val["dtype"]])
+    # Operands that take a result: the program's own decision, less the inputs that must stay.
+    protected = {prog.inputs[i] for i in protected_inputs}
+    root_of = StorageUse(g, prog.instrs, prog.inputs, prog.outputs).root
+    takes_over = {(idx, v) for idx, v in prog.takes_over if root_of.get(v, v) not in protected}
     # Values whose storage a task output ends up naming - directly, through view-like operators
-    # (autograd hands saved tensors on as detached aliases) or because an operator may write its
+    # (autograd hands saved tensors on as detached aliases) or because an operator writes its
     # result over them - are placed in the output block from the start, so no output is copied.
     alias_parent: Dict[int, int] = {}
-    for ins in prog.instrs:
+    for idx, ins in enumerate(prog.instrs):
         if ins.kind == 1 and isinstance(ins.args, int):
             alias_parent[ins.outs[0]] = ins.args
         elif ins.kind in (0, 6):
@@ -743,8 +719,8 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
             ids_ = _tensor_ids_in_order(ins.args, ins.kwargs)
             if EMITTERS.get(opn) in (_emit_view, _emit_alias) and ids_:
                 alias_parent[ins.outs[0]] = ids_[0]
-            for operand, result in _MAY_WRITE_OVER.get(opn, ()):
-                if operand < len(ids_) and result < len(ins.outs):
+            for operand, result in MAY_WRITE_OVER.get(opn, ()):
+                if operand < len(ids_) and result < len(ins.outs) and (idx, ids_[operand]) in takes_over:
                     alias_parent[ins.outs[result]] = ids_[operand]
     b.reaches_output = {v for k, v in enumerate(prog.outputs) if accumulate[k] == 0}
     for ins in reversed(prog.instrs):
@@ -768,27 +744,7 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
             alone = readers.get(v, 0) == 1 and v not in prog.outputs
         if alone and plan_store_dtype(plan, template, k) == "float32":
             b.sole_accumulator[v] = k
-    # operand liveness inside the program, and operands other tasks still need
-    last: Dict[int, int] = {}
-    for idx, ins in enumerate(prog.instrs):
-        for v in _reads_of(ins):
-            last[v] = idx
-    keep = set(prog.outputs)
-    mine = set(prog.inputs)
-    shared_inputs = {v for t in plan["templates"] if t is not template and t["name"] != template["name"]
-                     for v in t["inputs"] if v in mine}
-    shared_inputs |= {prog.inputs[i] for i in protected_inputs}
-
-    def may_overwrite(ins: Instr, vid: int) -> bool:
-        """The operand dies with this instruction and its storage may take the result (the rule
-        of the interpreted program's in-place operator variants)."""
-        idx = b.cur
-        if last.get(vid, -1) > idx or vid in keep or vid in shared_inputs:
-            return False
-        if vid in b.scaled:
-            return False
-        return True       # input tiles are private to the step (non-donated arguments are cloned when bound)
-    b.may_overwrite = may_overwrite
+    b.may_overwrite = lambda ins, vid: (b.cur, vid) in takes_over and vid not in b.scaled
 
     for idx, ins in enumerate(prog.instrs):
         b.cur = idx

@@ -334,13 +334,13 @@ _define("embedding_bwd(Tensor dout, Tensor ids, int vocab) -> Tensor", embedding
 
 # ------------------------------------------------------------------------- adamw
 def adamw_impl(param, master, m, v, grad, step, lr: float, beta1: float, beta2: float, eps: float, wd: float,
-               grad_scale: float, inplace: bool = False):
-    """One AdamW update. Returns (working copy, master, m, v). ``param`` is the current
-    working copy (its buffer is reused when ``inplace``); ``step`` is a 1-element int64
+               grad_scale: float, overwrite=(False, False, False, False)):
+    """One AdamW update. Returns (working copy, master, m, v), written over the first four
+    operands where ``overwrite`` says so; ``step`` is a 1-element int64
     tensor on the same device holding the step count *after* this update (the kernel
     reads it, so the update never synchronises with the host)."""
-    if not inplace:
-        param, master, m, v = torch.empty_like(param), master.clone(), m.clone(), v.clone()
+    param = param if overwrite[0] else torch.empty_like(param)
+    master, m, v = (t if over else t.clone() for t, over in zip((master, m, v), overwrite[1:]))
     g = grad.reshape(-1)
     if g.dtype != torch.float32:
         g = g.float()
@@ -354,7 +354,7 @@ def adamw_impl(param, master, m, v, grad, step, lr: float, beta1: float, beta2: 
 _define("adamw(Tensor param, Tensor master, Tensor m, Tensor v, Tensor grad, Tensor step, float lr, float beta1,"
         " float beta2, float eps, float wd, float grad_scale) -> (Tensor, Tensor, Tensor, Tensor)",
         lambda param, master, m, v, grad, step, lr, beta1, beta2, eps, wd, gs: adamw_impl(
-            param, master, m, v, grad, step, lr, beta1, beta2, eps, wd, gs, False),
+            param, master, m, v, grad, step, lr, beta1, beta2, eps, wd, gs),
         lambda param, master, m, v, grad, step, lr, beta1, beta2, eps, wd, gs: (
             torch.empty_like(param), torch.empty_like(master), torch.empty_like(m), torch.empty_like(v)))
 
@@ -523,8 +523,8 @@ def _cross_entropy_fast(logits, targets, scale):
     return cross_entropy_impl(logits, targets, scale, inplace=True)
 
 
-def _adamw_fast(param, master, m, v, grad, step, lr, beta1, beta2, eps, wd, gs):
-    return adamw_impl(param, master, m, v, grad, step, lr, beta1, beta2, eps, wd, gs, inplace=True)
+def _adamw_fast(param, master, m, v, grad, step, lr, beta1, beta2, eps, wd, gs, overwrite=(True, True, True, True)):
+    return adamw_impl(param, master, m, v, grad, step, lr, beta1, beta2, eps, wd, gs, overwrite=overwrite)
 
 
 FAST_OPS: Dict[str, object] = {
@@ -544,11 +544,14 @@ FAST_OPS: Dict[str, object] = {
     "mm_ops.embedding_bwd.default": embedding_bwd_fast,
     "mm_ops.adamw.default": _adamw_fast,
 }
-# tensor operands (by position among the tensor arguments) that the fast variant overwrites
-INPLACE_OPERANDS: Dict[str, tuple] = {
-    "mm_ops.add_rmsnorm_bwd.default": (2,),
-    "mm_ops.attention.default": (0,),
-    "mm_ops.cross_entropy.default": (0,),
+# operators that may write a result over an operand that nothing needs any more: (position among the
+# tensor operands, result position). The fast variants above and the native task programs do so.
+MAY_WRITE_OVER: Dict[str, tuple] = {
+    "mm_ops.attention.default": ((0, 2),),
+    "mm_ops.add_rmsnorm_bwd.default": ((2, 0),),
+    "mm_ops.cross_entropy.default": ((0, 1),),
+    "mm_ops.adamw.default": ((0, 0), (1, 1), (2, 2), (3, 3)),
+    "aten.mul.Tensor": ((0, 0),),
 }
 # operators whose fast variant can write into a gradient accumulator (acc=(buffer|None, dtype))
 ACC_FUSABLE = {"mm_ops.linear_wgrad.default", "mm_ops.embedding_bwd.default"}

@@ -21,7 +21,7 @@ from torch.utils import _pytree as pytree
 
 from .. import state
 from ..compiler.capture import Captured, DTYPE_FROM_NAME
-from ..compiler.lower import TemplateProgram, build_program
+from ..compiler.lower import TemplateProgram, build_program, overwritable_inputs
 from ..ops import kernels as K
 from .collectives import DeviceCtx, Rendezvous, Topology, tile_box
 
@@ -157,10 +157,11 @@ class Executable:
         # sub-meshes per microbatch runs one template on several device ranges)
         runs_here = {op["template"] for op in plan["ops"] if op["kind"] == "task" and
                      any(topology.is_local(d) for d in range(op["device_start"], op["device_start"] + op["num_devices"]))}
+        overwritable = overwritable_inputs(cap, plan)
         for t in plan["templates"]:
             local = t["id"] in runs_here or any(topology.is_local(d) for d in self._template_devices(t))
             if local or topology.kind != "dist":
-                self.programs[t["id"]] = build_program(cap, plan, t, fast_ops, acc_fusable)
+                self.programs[t["id"]] = build_program(cap, plan, t, fast_ops, acc_fusable, overwritable)
         # A process that drives exactly one CUDA device gets the context that owns the device's
         # streams: tasks on the caller's compute stream, reshards and once-per-step collectives on
         # a communication stream, ordered by CUDA events wherever the dependence analysis finds a
@@ -254,6 +255,11 @@ class Executable:
                 self._dying_inputs.setdefault(k, set()).add(sid)
         self._build_native_programs()
         self._shared_params = self._find_shared_params()
+        written = {s for op in plan["ops"] if op["kind"] == "task" and op["template"] in self.programs
+                   for s, v in zip(op["inputs"], self.programs[op["template"]].inputs)
+                   if v in self.programs[op["template"]].written_inputs}
+        # arguments some task writes over: a private copy of those that were not donated
+        self._written_params = {i for i, sid in enumerate(plan["param_stores"]) if sid in written}
         # Debug aid for the compiler's buffer plan (MM_CHECK_LIFETIMES=1): stores that share a
         # physical buffer must never be alive at the same time. With the knob on, every tile
         # remembers which store wrote it last; a task or reshard that reads a store whose buffer
@@ -598,6 +604,8 @@ class Executable:
                 if a.sharding["key"] != want["key"]:
                     a = shard_tensor(a.full_tensor(), want, topo)
                 new_tiles = a.local_tiles()
+                if i in self._written_params and i not in self.donated:
+                    new_tiles = {d_: t.clone() for d_, t in new_tiles.items()}
             else:
                 new_tiles = shard_tensor(a, want, topo, private=i not in self.donated and i not in self._shared_params).local_tiles()
             self.tiles[sid].clear()
