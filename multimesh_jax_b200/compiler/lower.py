@@ -132,8 +132,10 @@ class TemplateProgram:
                 x = env[ins.args]
                 piece = x.narrow(dim, scalars[0] // shards, size // shards)
                 # rows of the leading dimension are one block of memory; a slice of an inner
-                # dimension is not, and the captured operators (views) expect a dense operand
-                env[ins.outs[0]] = piece if piece.is_contiguous() else piece.contiguous()
+                # dimension is not, and the captured operators (views) expect a dense operand; the
+                # kernels load 16 bytes at a time, and rows need not end on such a boundary
+                dense = piece.is_contiguous() and (piece.data_ptr() % 16 == 0 or not piece.is_floating_point())
+                env[ins.outs[0]] = piece if dense else piece.clone(memory_format=torch.contiguous_format)
             elif kind == 4:  # all-reduce over mesh axes
                 axes, scale, in_place = ins.extra
                 y = ctx.all_reduce(env[ins.args], axes, ins.node_id, in_place=in_place)

@@ -468,7 +468,8 @@ def _emit_attention_bwd(b: _Builder, ins: Instr, ids, op):
     dqkv = b.new_value(ins.outs[0], qkv_r.shape, qkv_r.dtype)
     dq_acc = b.temp((B, S, hq, D), torch.float32)
     rows = b.temp((b.lib.mm_flash_attn_bwd_rows(B, S, hq),), torch.float32)
-    fused = cos.shape == (S, D // 2) and cos.dtype == torch.float32
+    # (every slot starts on a 16-byte boundary, so the tables do)
+    fused = cos.shape == sin.shape == (S, D // 2) and cos.dtype == sin.dtype == torch.float32
     b.call("mm_flash_attn_bwd", qkv_r, out, dout, lse, dqkv, dq_acc, rows, cos if fused else None, sin if fused else None,
            B, S, hkv, rep, D, STREAM)
     b.free_temp(dq_acc)

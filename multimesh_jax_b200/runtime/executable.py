@@ -115,10 +115,17 @@ class ShardedTensor:
         return f"ShardedTensor({self.sharding['key']})"
 
 
+def vector_aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t``, or a copy of it when it does not start on the 16-byte boundary that the vector loads and tensor
+    maps of the kernels take for granted (a view into a flat buffer can start anywhere)."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def shard_tensor(t: torch.Tensor, sharding: dict, topology: Topology, private: bool = False) -> ShardedTensor:
     """Slices a global tensor into the tiles of ``sharding`` (local devices only). Tiles are
-    contiguous; with ``private`` they never share storage with ``t`` (needed for arguments
-    that were not donated, because compiled tasks may update dead inputs in place)."""
+    contiguous, but where they share storage with ``t`` they start wherever ``t`` does; with
+    ``private`` they never share it (needed for arguments that were not donated and that some
+    task may write over)."""
     tiles: Dict[int, torch.Tensor] = {}
     start = sharding["device_start"]
     seen_shared = False
@@ -609,7 +616,7 @@ class Executable:
             else:
                 new_tiles = shard_tensor(a, want, topo, private=i not in self.donated and i not in self._shared_params).local_tiles()
             self.tiles[sid].clear()
-            self.tiles[sid].update(new_tiles)
+            self.tiles[sid].update((d_, vector_aligned(t)) for d_, t in new_tiles.items())
             if self._lifetimes:
                 for d_ in new_tiles:
                     self._owner[(self.buffer_of[sid], d_)] = self._alias_root[sid]
@@ -845,6 +852,8 @@ class Executable:
                     o = ext_tiles[spec[1]].view(spec[2])
                 elif spec[0] == "slice":
                     o = ins[spec[1]].narrow(0, scalars[0], spec[2][0]).view(spec[2])
+                    if o.is_floating_point():       # (token ids are read one by one)
+                        o = vector_aligned(o)
                 else:
                     o = ins[spec[1]].view(spec[2])
                 if self._lifetimes:

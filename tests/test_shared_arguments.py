@@ -4,6 +4,7 @@ import torch
 from torch.utils import _pytree as pytree
 
 import multimesh_jax_b200 as mm
+from multimesh_jax_b200.compiler.lower import Instr, TemplateProgram
 from multimesh_jax_b200.compiler.native import inputs_left_alone
 from multimesh_jax_b200.models import llama
 
@@ -61,4 +62,60 @@ def test_shared_arguments_keep_their_values_and_follow_updates():
     assert torch.equal(out, kept)
     args[0]["embed"].mul_(2.0)
     assert exe(*args)[0].full_tensor().item() != first
+    exe.shutdown()
+
+
+def _offset_view(t):
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    flat[1:] = t.reshape(-1)
+    return flat[1:].view(t.shape)
+
+
+@pytest.mark.parametrize("donate", [False, True])
+def test_tiles_of_arguments_start_on_vector_boundaries(donate):
+    exe, args = _loss_step("cpu", train=donate)
+    exe._shared_params = set(range(len(exe.plan["param_stores"])))      # as on a device: nothing is copied for privacy
+    exe.donated = set(exe._shared_params) if donate else set()
+    want = exe(*pytree.tree_map(torch.clone, args))[0].full_tensor()
+    odd = pytree.tree_map(_offset_view, args)
+    even = pytree.tree_map(torch.clone, args)
+    assert any(t.data_ptr() % 16 for t in pytree.tree_leaves(odd))
+    for call in (odd, even):
+        bound = {}
+        bind = exe._submit_task
+
+        def first_task(k, op, d, *rest):
+            bound.update({sid: exe.tiles[sid][0] for sid in exe.plan["param_stores"] if sid >= 0 and not bound.get(sid) is not None
+                          and 0 in exe.tiles[sid]})
+            return bind(k, op, d, *rest)
+
+        exe._submit_task = first_task
+        loss = exe(*call)[0].full_tensor()
+        exe._submit_task = bind
+        assert torch.equal(loss, want)
+        leaves = pytree.tree_leaves(call)
+        for i, sid in enumerate(exe.plan["param_stores"]):
+            if sid >= 0:
+                assert bound[sid].data_ptr() % 16 == 0
+                assert (bound[sid].data_ptr() == leaves[i].data_ptr()) == (leaves[i].data_ptr() % 16 == 0)
+    exe.shutdown()
+
+
+def test_microbatch_slices_start_on_vector_boundaries():
+    prog = TemplateProgram({"name": "t", "mesh_dims": [1], "device_start": 0}, [Instr(3, None, 0, None, [1], None, 0, (0, 1, 1))],
+                           [0], [1], {})
+    for x in (torch.randn(6, 12).bfloat16(), torch.randn(6, 8).bfloat16(), torch.arange(6).view(6, 1)):
+        for row in range(6):
+            (piece,) = prog.run(None, [row], [x])
+            assert torch.equal(piece, x[row:row + 1])
+            assert piece.data_ptr() % 16 == 0 or not piece.is_floating_point()
+            # rows that start well, and token ids wherever they start, stay in the argument's memory
+            assert (piece.data_ptr() == x[row].data_ptr()) == (x[row].data_ptr() % 16 == 0 or not x.is_floating_point())
+
+
+@pytest.mark.gpu
+def test_arguments_at_odd_offsets_on_the_device():
+    exe, args = _loss_step("cuda", train=False)
+    want = exe(*args)[0].full_tensor()
+    assert torch.equal(exe(*pytree.tree_map(_offset_view, args))[0].full_tensor(), want)
     exe.shutdown()
