@@ -13,6 +13,8 @@ from __future__ import annotations
 
 from typing import Any, Dict, List, Optional, Tuple
 
+import functools
+import operator
 import os
 import threading
 
@@ -115,10 +117,9 @@ class ShardedTensor:
         return f"ShardedTensor({self.sharding['key']})"
 
 
-def vector_aligned(t: torch.Tensor) -> torch.Tensor:
-    """``t``, or a copy of it when it does not start on the 16-byte boundary that the vector loads and tensor
-    maps of the kernels take for granted (a view into a flat buffer can start anywhere)."""
-    return t if t.data_ptr() % 16 == 0 else t.clone()
+# Vector loads and tensor maps of the kernels take tiles for granted that start on such a boundary; a view
+# into a flat buffer can start anywhere and is copied.
+VECTOR_BYTES = 16
 
 
 def shard_tensor(t: torch.Tensor, sharding: dict, topology: Topology, private: bool = False) -> ShardedTensor:
@@ -267,6 +268,18 @@ class Executable:
                    if v in self.programs[op["template"]].written_inputs}
         # arguments some task writes over: a private copy of those that were not donated
         self._written_params = {i for i, sid in enumerate(plan["param_stores"]) if sid in written}
+        # of the local tiles of every argument, in order: size, and whether some task writes over it
+        self._param_bytes: List[int] = []
+        self._param_written: List[bool] = []
+        for sid in plan["param_stores"]:
+            if sid >= 0:
+                shape = plan["stores"][sid]["shape"]
+                n = DTYPE_FROM_NAME[shape["dtype"]].itemsize
+                for e in shape["shard_size"]:
+                    n *= e
+                local = sum(topology.is_local(shape["device_start"] + o) for o in range(shape["num_devices"]))
+                self._param_bytes += [n] * local
+                self._param_written += [sid in written] * local
         # Debug aid for the compiler's buffer plan (MM_CHECK_LIFETIMES=1): stores that share a
         # physical buffer must never be alive at the same time. With the knob on, every tile
         # remembers which store wrote it last; a task or reshard that reads a store whose buffer
@@ -309,6 +322,43 @@ class Executable:
             kept |= {s for s, v in zip(op["inputs"], prog.inputs) if not plain or v not in clean[op["template"]]}
             kept |= set(op["outputs"])
         return {i for i, sid in enumerate(plan["param_stores"]) if sid >= 0 and sid not in kept}
+
+    def _copy_where_needed(self, bound: List[Tuple[int, int, Dict[int, torch.Tensor]]]) -> None:
+        """Replaces tiles of the step's arguments, given as (argument, store, tiles per device), by copies:
+
+        * a tile that does not start on a ``VECTOR_BYTES`` boundary;
+        * where a task writes over an argument, the other arguments in its memory - one tensor may be passed
+          several times, or as views that overlap - so that they keep the values they were passed with."""
+        ptrs = [t.data_ptr() for _, _, tiles in bound for t in tiles.values()]
+        if functools.reduce(operator.or_, ptrs, 0) % VECTOR_BYTES == 0:
+            if not self._written_params:
+                return
+            end, clash = 0, False
+            for start, nbytes, written in sorted(zip(ptrs, self._param_bytes, self._param_written)):
+                if start >= end:
+                    clash = written
+                elif clash or written:
+                    break
+                end = max(end, start + nbytes)
+            else:
+                return
+        for _, _, tiles in bound:
+            for d, t in tiles.items():
+                if t.data_ptr() % VECTOR_BYTES:
+                    tiles[d] = t.clone()
+        spans = sorted((t.data_ptr(), t.data_ptr() + t.nbytes, k, d)
+                       for k, (_, _, tiles) in enumerate(bound) for d, t in tiles.items() if t.numel())
+        group: List[Tuple[int, int]] = []
+        end = 0
+        for start, stop, k, d in spans + [(1 << 64, 1 << 64, -1, -1)]:
+            if start >= end:            # nothing so far reaches into this span
+                keep = next((g for g in group if bound[g[0]][0] in self._written_params), None)
+                for g in group if keep is not None else ():
+                    if g != keep:
+                        bound[g[0]][2][g[1]] = bound[g[0]][2][g[1]].clone()
+                group = []
+            group.append((k, d))
+            end = max(end, stop)
 
     def _took_buffer(self, sid: int, d: int, old: Optional[torch.Tensor], new: torch.Tensor) -> None:
         """Store ``sid`` has just been written on device ``d`` (lifetime checking only)."""
@@ -602,6 +652,7 @@ class Executable:
                         ctx.create_store(self.buffer_of[st["id"]], d, nbytes, False)
             self._created = True
         # parameter stores
+        bound: List[Tuple[int, int, Dict[int, torch.Tensor]]] = []
         for i, sid in enumerate(plan["param_stores"]):
             if sid < 0:
                 continue
@@ -615,8 +666,11 @@ class Executable:
                     new_tiles = {d_: t.clone() for d_, t in new_tiles.items()}
             else:
                 new_tiles = shard_tensor(a, want, topo, private=i not in self.donated and i not in self._shared_params).local_tiles()
+            bound.append((i, sid, new_tiles))
+        self._copy_where_needed(bound)
+        for _, sid, new_tiles in bound:
             self.tiles[sid].clear()
-            self.tiles[sid].update((d_, vector_aligned(t)) for d_, t in new_tiles.items())
+            self.tiles[sid].update(new_tiles)
             if self._lifetimes:
                 for d_ in new_tiles:
                     self._owner[(self.buffer_of[sid], d_)] = self._alias_root[sid]
@@ -852,8 +906,8 @@ class Executable:
                     o = ext_tiles[spec[1]].view(spec[2])
                 elif spec[0] == "slice":
                     o = ins[spec[1]].narrow(0, scalars[0], spec[2][0]).view(spec[2])
-                    if o.is_floating_point():       # (token ids are read one by one)
-                        o = vector_aligned(o)
+                    if o.data_ptr() % VECTOR_BYTES and o.is_floating_point():       # (token ids are read one by one)
+                        o = o.clone()
                 else:
                     o = ins[spec[1]].view(spec[2])
                 if self._lifetimes:

@@ -119,3 +119,29 @@ def test_arguments_at_odd_offsets_on_the_device():
     want = exe(*args)[0].full_tensor()
     assert torch.equal(exe(*pytree.tree_map(_offset_view, args))[0].full_tensor(), want)
     exe.shutdown()
+
+
+def test_one_tensor_passed_as_a_written_and_as_a_read_argument():
+    """AdamW writes over donated state; another argument in the same memory keeps what it was passed with."""
+    ops = torch.ops.mm_ops
+    torch.manual_seed(0)
+    p, g, t = torch.randn(64).bfloat16(), torch.randn(64), torch.tensor([3])
+    flat = torch.randn(192).abs()
+
+    def step(p, master, m, v, g, t, ref):
+        new = ops.adamw(p, master, m, v, g, t, 1e-2, 0.9, 0.95, 1e-8, 0.1, 1.0)
+        return (*new, new[1] - ref)
+
+    with mm.enable_fast_path(False):
+        exe = mm.compile_function(step, (p, *[flat[:64]] * 3, g, t, flat[:64]), num_devices=1, backend="cpu",
+                                  donate_argnums=(0, 1, 2, 3))
+    exe._shared_params = {4, 5, 6}      # as on a device
+    # (master, m, v, ref): apart; ref is the master; ref lies across two of them; both moments and ref are one tensor
+    for spans in ((0, 64, 128, None), (0, 64, 128, 0), (0, 64, 128, 32), (0, 64, 64, 64), (0, 0, 0, 0)):
+        memory = flat.clone()
+        parts = [memory[s:s + 64] if s is not None else flat[3:67].clone() for s in spans]
+        want = step(p, *(x.clone() for x in parts[:3]), g, t, parts[3].clone())
+        got = exe(p.clone(), *parts[:3], g, t, parts[3])
+        for a, b in zip(got, want):
+            assert torch.equal(a.full_tensor(), b), spans
+    exe.shutdown()
