@@ -712,14 +712,15 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
     # (autograd hands saved tensors on as detached aliases) or because an operator writes its
     # result over them - are placed in the output block from the start, so no output is copied.
     alias_parent: Dict[int, int] = {}
+    same_value: Dict[int, int] = {}         # the views and identities alone
     for idx, ins in enumerate(prog.instrs):
         if ins.kind == 1 and isinstance(ins.args, int):
-            alias_parent[ins.outs[0]] = ins.args
+            alias_parent[ins.outs[0]] = same_value[ins.outs[0]] = ins.args
         elif ins.kind in (0, 6):
             opn = g.node(ins.node_id)["op"]
             ids_ = _tensor_ids_in_order(ins.args, ins.kwargs)
             if EMITTERS.get(opn) in (_emit_view, _emit_alias) and ids_:
-                alias_parent[ins.outs[0]] = ids_[0]
+                alias_parent[ins.outs[0]] = same_value[ins.outs[0]] = ids_[0]
             for operand, result in MAY_WRITE_OVER.get(opn, ()):
                 if operand < len(ids_) and result < len(ins.outs) and (idx, ids_[operand]) in takes_over:
                     alias_parent[ins.outs[result]] = ids_[operand]
@@ -740,8 +741,8 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
         if not accumulate[k] or k in prog.fused_acc or prog.outputs.count(v) > 1:
             continue
         alone = readers.get(v, 0) == 0
-        while v in alias_parent and alone:
-            v = alias_parent[v]
+        while v in same_value and alone:
+            v = same_value[v]
             alone = readers.get(v, 0) == 1 and v not in prog.outputs
         if alone and plan_store_dtype(plan, template, k) == "float32":
             b.sole_accumulator[v] = k

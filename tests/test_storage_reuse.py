@@ -26,6 +26,13 @@ def _cross_entropy(m, buf, targets, loss, _, __, rows, V, ___, ____, scale, grad
     m(loss).copy_(K.cross_entropy_fwd_bwd(m(buf).view(rows, V), m(targets).reshape(-1), scale, bool(grad)))
 
 
+def _norm_bwd(m, x, w, dy, rstd, dx, dw, accumulate, add):
+    assert not add
+    got, d = K.rmsnorm_bwd(m(x), m(w), m(dy), m(rstd))
+    m(dx).copy_(got)
+    m(dw).copy_((m(dw) if accumulate else 0) + d.bfloat16().float())
+
+
 REPLAY = {
     "mm_gemm_auto_bf16": _gemm,
     "mm_cross_entropy": _cross_entropy,
@@ -36,6 +43,10 @@ REPLAY = {
     "mm_bf16_to_f32": lambda m, x, out, n, acc, *_: m(out).copy_(m(x).float().view(out.shape) + (m(out) if acc else 0)),
     "mm_embedding_fwd": lambda m, table, tok, out, *_: m(out).copy_(m(table)[m(tok)]),
     "mm_accumulate_f32": lambda m, acc, x, *_: m(acc).add_(m(x).view(acc.shape)),
+    "mm_rmsnorm_fwd": lambda m, x, w, y, rstd, rows, D, eps, *_: [m(o).copy_(r.view(o.shape)) for o, r in zip(
+        (y, rstd), K.rmsnorm_fwd(m(x), m(w), eps))],
+    "mm_rmsnorm_bwd_bf16": lambda m, *a: _norm_bwd(m, *a[:6], 0, 0),
+    "mm_rmsnorm_bwd_acc": lambda m, *a: _norm_bwd(m, *a[:6], a[9], a[10]),
     "mm_sum_scale_f32": lambda m, x, n, scale, out, *_: m(out).copy_(m(x).sum() * scale),
 }
 
@@ -167,6 +178,30 @@ def test_loop_invariant_argument_is_scaled_once_per_microbatch(monkeypatch):
     torch.testing.assert_close(got, want.float(), rtol=1e-5, atol=1e-5)     # fp32 sums of four losses
     assert all(torch.equal(kept[sid], a) for sid, a in zip(exe.plan["param_stores"], (w, s)))
     torch.testing.assert_close(exe(w, s, x, t).full_tensor(), want.float(), rtol=1e-5, atol=1e-5)
+    exe.shutdown()
+
+
+@pytest.mark.parametrize("scaled", [False, True])
+def test_norm_weight_gradient_scaled_before_it_is_accumulated(scaled, monkeypatch):
+    torch.manual_seed(5)
+    table, w, s, tokens = _b(32, 64), torch.rand(64).bfloat16(), torch.tensor([0.5]).bfloat16(), torch.randint(0, 32, (8,))
+
+    def step(table, w, s, tokens):
+        def gradient(w, batch):
+            x = ops.embedding(table, batch)
+            y, rstd = ops.rmsnorm(x, w, 1e-5)
+            dw = ops.rmsnorm_bwd(x, w, y, rstd)[1]
+            return dw * s if scaled else dw
+        return mm.microbatch(gradient, size=2, argnum=1, accumulate_dtype=torch.float32)(w, tokens)
+
+    args = (table, w, s, tokens)
+    want = sum(step_part.float() for step_part in (
+        (lambda x: ops.rmsnorm_bwd(x, w, *ops.rmsnorm(x, w, 1e-5))[1] * (s if scaled else 1))(ops.embedding(table, tokens[i:i + 2]))
+        for i in range(0, 8, 2)))
+    exe = _compile(step, args)
+    (got,), _ = _replay(exe, args, monkeypatch)
+    assert torch.equal(got, want)
+    assert torch.equal(exe(*args).full_tensor(), want)
     exe.shutdown()
 
 
