@@ -802,7 +802,7 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
                     b.np.outputs.append(("acc", k))
                 else:
                     fr = b.fresh_acc[k]
-                    b.np.outputs.append(("block", b.out_chunk_of(fr.slot), fr.off, fr.shape, fr.dtype))
+                    b.np.outputs.append(("block", b.out_chunk_of(fr.slot), fr.off, sym.shape, fr.dtype))
                 continue
             acc_dtype = DTYPE_FROM_NAME[plan_store_dtype(plan, template, k)]
             if acc_dtype != torch.float32:

@@ -181,8 +181,8 @@ def test_loop_invariant_argument_is_scaled_once_per_microbatch(monkeypatch):
     exe.shutdown()
 
 
-@pytest.mark.parametrize("scaled", [False, True])
-def test_norm_weight_gradient_scaled_before_it_is_accumulated(scaled, monkeypatch):
+@pytest.mark.parametrize("form", ["plain", "scaled", "other shape"])
+def test_norm_weight_gradient_on_its_way_into_the_accumulator(form, monkeypatch):
     torch.manual_seed(5)
     table, w, s, tokens = _b(32, 64), torch.rand(64).bfloat16(), torch.tensor([0.5]).bfloat16(), torch.randint(0, 32, (8,))
 
@@ -191,13 +191,13 @@ def test_norm_weight_gradient_scaled_before_it_is_accumulated(scaled, monkeypatc
             x = ops.embedding(table, batch)
             y, rstd = ops.rmsnorm(x, w, 1e-5)
             dw = ops.rmsnorm_bwd(x, w, y, rstd)[1]
-            return dw * s if scaled else dw
+            return dw * s if form == "scaled" else dw.view(8, 8) if form == "other shape" else dw
         return mm.microbatch(gradient, size=2, argnum=1, accumulate_dtype=torch.float32)(w, tokens)
 
     args = (table, w, s, tokens)
     want = sum(step_part.float() for step_part in (
-        (lambda x: ops.rmsnorm_bwd(x, w, *ops.rmsnorm(x, w, 1e-5))[1] * (s if scaled else 1))(ops.embedding(table, tokens[i:i + 2]))
-        for i in range(0, 8, 2)))
+        (lambda x: ops.rmsnorm_bwd(x, w, *ops.rmsnorm(x, w, 1e-5))[1] * (s if form == "scaled" else 1))(ops.embedding(table, tokens[i:i + 2]))
+        for i in range(0, 8, 2))).view((8, 8) if form == "other shape" else (64,))
     exe = _compile(step, args)
     (got,), _ = _replay(exe, args, monkeypatch)
     assert torch.equal(got, want)
