@@ -427,6 +427,18 @@ int64_t mm_moe_workspace(int T, int D, int F, int E, int k, int backward) {
   return MoeSpace(nullptr, T, D, F, E, k, backward != 0).used;
 }
 
+// The router alone: the k experts of every token and their gates, as the two passes below choose them.
+// x [T, D], wr [E, D] bf16, contiguous and 16-byte aligned; idx, gates [T, k].
+int mm_moe_route(const void* x, const void* wr, int* idx, float* gates, int T, int D, int E, int k, cudaStream_t stream) {
+  using namespace mm;
+  const int rc = moe_check(T, D, 8, E, k);
+  if (rc) return rc;
+  ml_route_kernel<<<(T + ML_TOK - 1) / ML_TOK, 128, 0, stream>>>(static_cast<const __nv_bfloat16*>(x),
+                                                                static_cast<const __nv_bfloat16*>(wr), T, D, E, k, idx, gates);
+  MM_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
 // y[T, D] = sum over the k chosen experts of gate * W_down (silu(W_gate x) * W_up x). All tensors bf16,
 // contiguous and 16-byte aligned: x [T, D], wr [E, D], wgu [E, 2, F, D], wdown [E, D, F]; ws: 256-byte aligned.
 int mm_moe_fwd(const void* x, const void* wr, const void* wgu, const void* wdown, void* y, void* ws, int T, int D, int F, int E,

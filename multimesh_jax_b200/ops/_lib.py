@@ -30,6 +30,7 @@ _SIGS = {
     "mm_gemm_pair_dyn_bf16": (c_int, [_P, c_int, c_int64, _P, c_int, c_int64, _P, c_int, c_int64,
                                       c_int, c_int, c_int, _P, _P, _P]),
     "mm_moe_workspace": (c_int64, [c_int] * 6),
+    "mm_moe_route": (c_int, [_P] * 4 + [c_int] * 4 + [_P]),
     "mm_moe_fwd": (c_int, [_P] * 6 + [c_int] * 5 + [_P]),
     "mm_moe_bwd": (c_int, [_P] * 10 + [c_int] * 5 + [_P]),
     "mm_zero_row_tail": (c_int, [_P, c_int64, _P, c_int, c_int, _P]),

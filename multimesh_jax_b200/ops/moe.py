@@ -108,14 +108,13 @@ def _expert_bwd(rows, d_out, wgu_e, wdown_e, dx_out=None, out=None, count=None, 
 # --------------------------------------------------------------------------- global view
 # The one-launch-per-step form keeps the activations of all experts at once where the loop over the
 # experts keeps those of one. Above this much workspace the loop runs: the GEMMs are then long enough
-# to hide its launches and host reads (4096 tokens of a Mixtral block take 1.3 GB).
+# to hide its launches and host reads (4096 tokens of a Mixtral block take 0.9 GB forward, 1.0 GB backward).
 GROUPED_WORKSPACE_LIMIT = 8 << 30
 
 
 def _grouped_workspace(x2, wr, wgu, wdown, top_k: int, backward: bool):
-    """Bytes of workspace when the block can run on the grouped kernels, else ``None``: CUDA, all four
-    operands bf16 on one device, sizes that the kernels take (D and F multiples of 8, at most 64 experts,
-    at most 4 choices), workspace below :data:`GROUPED_WORKSPACE_LIMIT`."""
+    """Bytes of workspace of the grouped kernels, or ``None`` where they do not take the block: CUDA, all
+    four operands bf16 on one device, D and F multiples of 8, at most 64 experts, at most 4 choices."""
     E, _, F, D = wgu.shape
     if not x2.is_cuda or any(t.dtype != torch.bfloat16 or t.device != x2.device for t in (x2, wr, wgu, wdown)):
         return None
@@ -124,7 +123,27 @@ def _grouped_workspace(x2, wr, wgu, wdown, top_k: int, backward: bool):
     if x2.shape[0] * top_k >= 1 << 30:
         return None
     need = _lib.load().mm_moe_workspace(x2.shape[0], D, F, E, top_k, int(backward))
-    return need if 0 <= need <= GROUPED_WORKSPACE_LIMIT else None
+    return need if need >= 0 else None
+
+
+def _workspace(nbytes: int, device):
+    """Workspace of the grouped kernels, or ``None`` - the loop runs - above the limit."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes <= GROUPED_WORKSPACE_LIMIT else None
+
+
+def _route_as_grouped(x2: torch.Tensor, wr: torch.Tensor, top_k: int) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Chosen experts and gates from the router of the grouped kernels. The loop takes it wherever those
+    kernels could have run, because the two passes of one block may run in different forms: sums in
+    another order choose other experts for tokens whose logits are nearly equal."""
+    x2, wr = _packed(x2), _packed(wr)
+    T, D = x2.shape
+    idx = torch.empty(T, top_k, dtype=torch.int32, device=x2.device)
+    gates = torch.empty(T, top_k, dtype=torch.float32, device=x2.device)
+    rc = _lib.load().mm_moe_route(x2.data_ptr(), wr.data_ptr(), idx.data_ptr(), gates.data_ptr(), T, D, wr.shape[0], top_k,
+                                  K._stream())
+    _lib.check(rc, "mm_moe_route")
+    K._count()
+    return idx.long(), gates
 
 
 def _packed(t: torch.Tensor) -> torch.Tensor:
@@ -137,17 +156,17 @@ def moe_ffn_impl(x, wr, wgu, wdown, top_k: int):
     D = x.shape[-1]
     x2 = x.reshape(-1, D)
     need = _grouped_workspace(x2, wr, wgu, wdown, top_k, False)
-    if need is not None:
+    ws = _workspace(need, x.device) if need is not None else None
+    if ws is not None:
         x2, wr, wgu, wdown = (_packed(t) for t in (x2, wr, wgu, wdown))
         y = torch.empty_like(x2)
-        ws = torch.empty(need, dtype=torch.uint8, device=x.device)
         E, _, F, _ = wgu.shape
         rc = _lib.load().mm_moe_fwd(x2.data_ptr(), wr.data_ptr(), wgu.data_ptr(), wdown.data_ptr(), y.data_ptr(),
                                     ws.data_ptr(), x2.shape[0], D, F, E, top_k, K._stream())
         _lib.check(rc, "mm_moe_fwd")
         K._count(7)
         return y.view(x.shape)
-    _, topi, gates = route(x2, wr, top_k)
+    topi, gates = _route_as_grouped(x2, wr, top_k) if need is not None else route(x2, wr, top_k)[1:]
     y = torch.zeros(x2.shape, dtype=torch.float32, device=x.device)
     for e in range(wgu.shape[0]):
         hit = topi == e
@@ -163,11 +182,11 @@ def moe_ffn_impl(x, wr, wgu, wdown, top_k: int):
 def moe_ffn_bwd_impl(dy, x, wr, wgu, wdown, top_k: int):
     D = x.shape[-1]
     x2, dy2 = x.reshape(-1, D), dy.reshape(-1, D)
-    need = _grouped_workspace(x2, wr, wgu, wdown, top_k, True) if dy.dtype == x.dtype and dy.device == x.device else None
-    if need is not None:
+    need = _grouped_workspace(x2, wr, wgu, wdown, top_k, True)
+    ws = _workspace(need, x.device) if need is not None and dy.dtype == x.dtype and dy.device == x.device else None
+    if ws is not None:
         dy2, x2, wr, wgu, wdown = (_packed(t) for t in (dy2, x2, wr, wgu, wdown))
         dx, dwr, dwgu, dwdown = (torch.empty_like(t) for t in (x2, wr, wgu, wdown))
-        ws = torch.empty(need, dtype=torch.uint8, device=x.device)
         E, _, F, _ = wgu.shape
         rc = _lib.load().mm_moe_bwd(dy2.data_ptr(), x2.data_ptr(), wr.data_ptr(), wgu.data_ptr(), wdown.data_ptr(),
                                     dx.data_ptr(), dwr.data_ptr(), dwgu.data_ptr(), dwdown.data_ptr(), ws.data_ptr(),
@@ -175,7 +194,7 @@ def moe_ffn_bwd_impl(dy, x, wr, wgu, wdown, top_k: int):
         _lib.check(rc, "mm_moe_bwd")
         K._count(12)
         return dx.view(x.shape), dwr, dwgu, dwdown
-    _, topi, gates = route(x2, wr, top_k)
+    topi, gates = _route_as_grouped(x2, wr, top_k) if need is not None else route(x2, wr, top_k)[1:]
     dx = torch.zeros(x2.shape, dtype=torch.float32, device=x.device)
     dgates = torch.zeros_like(gates)
     dwgu = torch.zeros(wgu.shape, dtype=torch.float32, device=x.device)
