@@ -127,8 +127,14 @@ def _grouped_workspace(x2, wr, wgu, wdown, top_k: int, backward: bool):
 
 
 def _workspace(nbytes: int, device):
-    """Workspace of the grouped kernels, or ``None`` - the loop runs - above the limit."""
-    return torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes <= GROUPED_WORKSPACE_LIMIT else None
+    """Workspace of the grouped kernels, or ``None`` - the loop runs - above the limit and when the device
+    has no such block of memory."""
+    if nbytes > GROUPED_WORKSPACE_LIMIT:
+        return None
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
 
 
 def _route_as_grouped(x2: torch.Tensor, wr: torch.Tensor, top_k: int) -> Tuple[torch.Tensor, torch.Tensor]:
