@@ -188,6 +188,8 @@ def moe_ffn_impl(x, wr, wgu, wdown, top_k: int):
 def moe_ffn_bwd_impl(dy, x, wr, wgu, wdown, top_k: int):
     D = x.shape[-1]
     x2, dy2 = x.reshape(-1, D), dy.reshape(-1, D)
+    if dy2.shape != x2.shape:       # a row of dy is read for every row of x
+        raise ValueError(f"gradient of shape {tuple(dy.shape)} for an input of shape {tuple(x.shape)}")
     need = _grouped_workspace(x2, wr, wgu, wdown, top_k, True)
     ws = _workspace(need, x.device) if need is not None and dy.dtype == x.dtype and dy.device == x.device else None
     if ws is not None:

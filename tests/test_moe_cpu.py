@@ -137,3 +137,11 @@ def test_expert_functions_with_a_row_count_equal_the_exact_size_call(count):
     torch.testing.assert_close(dx[:count], ref_dx, rtol=1e-4, atol=1e-5)
     torch.testing.assert_close(dwgu, ref_dwgu, rtol=1e-4, atol=1e-5)
     torch.testing.assert_close(dwdown, ref_dwdown, rtol=1e-4, atol=1e-5)
+
+
+def test_gradient_with_fewer_rows_than_the_input_is_refused():
+    x, wr, wgu, wdown = torch.randn(6, 8), torch.randn(4, 8), torch.randn(4, 2, 8, 8), torch.randn(4, 8, 8)
+    with pytest.raises(ValueError, match="gradient of shape"):
+        torch.ops.mm_ops.moe_ffn_bwd(torch.randn(5, 8), x, wr, wgu, wdown, 2)
+    flat = torch.ops.mm_ops.moe_ffn_bwd(torch.ones(6, 8), x.view(2, 3, 8), wr, wgu, wdown, 2)
+    assert flat[0].shape == (2, 3, 8)
