@@ -78,22 +78,25 @@ def attention_bwd_packed(dout: torch.Tensor, qkv: torch.Tensor, out: torch.Tenso
     """Gradient of :func:`attention_fwd_packed` with respect to the packed projection. ``rope``: the
     (cos, sin) tables whose rotation was applied to the query and key heads of ``qkv`` before; the
     gradient is then the one with respect to the projection before that rotation."""
-    if rope is not None and not fuses_rope(qkv, dout, *rope):
-        B, S, H, D = qkv.shape
+    B, S, H, D = qkv.shape
+    hkv = H // (rep + 2)
+    hq = hkv * rep
+    if not (dout.numel() == out.numel() == B * S * hq * D and lse.numel() == B * hq * S):
+        raise ValueError(f"attention gradient: a projection of shape {tuple(qkv.shape)} has results of shape {(B, S, hq, D)} and "
+                         f"{(B, hq, S)}, got {tuple(dout.shape)}, {tuple(out.shape)} and {tuple(lse.shape)}")
+    native = native_supported(qkv) and dout.dtype == out.dtype == torch.bfloat16 and lse.dtype == torch.float32
+    if rope is not None and not (native and fuses_rope(qkv, dout, *rope)):
         dqkv = attention_bwd_packed(dout, qkv, out, lse, rep)
         K.rope_(dqkv.view(B * S, H, D), *rope, backward=True, rot_per_group=rep + 1, group_size=rep + 2)
         return dqkv
     dqkv = torch.empty_like(qkv)
-    if not (native_supported(qkv) and dout.dtype == torch.bfloat16):
+    if not native:
         q, k, v = _split_packed(qkv, rep)
         dq, dk, dv = _split_packed(dqkv, rep)
         attention_bwd(dout, q, k, v, out, lse, dq, dk, dv)
         return dqkv
-    B, S, H, D = qkv.shape
-    hkv = H // (rep + 2)
-    hq = hkv * rep
-    dout = dout.contiguous()
-    out = out.contiguous()
+    # the row statistics and the tensor map read dout and out 16 bytes at a time
+    dout, out, lse = K.packed(dout), K.packed(out), lse.contiguous()
     dq_acc = torch.empty((B, S, hq, D), dtype=torch.float32, device=qkv.device)
     lib = _lib.load()
     rows = torch.empty(lib.mm_flash_attn_bwd_rows(B, S, hq), dtype=torch.float32, device=qkv.device)

@@ -179,6 +179,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     return out
 
 
+def packed(t: torch.Tensor) -> torch.Tensor:
+    """The tensor itself when it is contiguous and 16-byte aligned, else such a copy."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def linear_fwd(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
                rows: Optional[torch.Tensor] = None) -> torch.Tensor:
     """y[T, N] = x[T, K] @ w[N, K]^T. ``rows``: device-side count of the rows of x that hold data."""

@@ -141,7 +141,7 @@ def _route_as_grouped(x2: torch.Tensor, wr: torch.Tensor, top_k: int) -> Tuple[t
     """Chosen experts and gates from the router of the grouped kernels. The loop takes it wherever those
     kernels could have run, because the two passes of one block may run in different forms: sums in
     another order choose other experts for tokens whose logits are nearly equal."""
-    x2, wr = _packed(x2), _packed(wr)
+    x2, wr = K.packed(x2), K.packed(wr)
     T, D = x2.shape
     idx = torch.empty(T, top_k, dtype=torch.int32, device=x2.device)
     gates = torch.empty(T, top_k, dtype=torch.float32, device=x2.device)
@@ -152,19 +152,13 @@ def _route_as_grouped(x2: torch.Tensor, wr: torch.Tensor, top_k: int) -> Tuple[t
     return idx.long(), gates
 
 
-def _packed(t: torch.Tensor) -> torch.Tensor:
-    """The tensor itself when it is contiguous and 16-byte aligned, else such a copy."""
-    t = t.contiguous()
-    return t if t.data_ptr() % 16 == 0 else t.clone()
-
-
 def moe_ffn_impl(x, wr, wgu, wdown, top_k: int):
     D = x.shape[-1]
     x2 = x.reshape(-1, D)
     need = _grouped_workspace(x2, wr, wgu, wdown, top_k, False)
     ws = _workspace(need, x.device) if need is not None else None
     if ws is not None:
-        x2, wr, wgu, wdown = (_packed(t) for t in (x2, wr, wgu, wdown))
+        x2, wr, wgu, wdown = (K.packed(t) for t in (x2, wr, wgu, wdown))
         y = torch.empty_like(x2)
         E, _, F, _ = wgu.shape
         rc = _lib.load().mm_moe_fwd(x2.data_ptr(), wr.data_ptr(), wgu.data_ptr(), wdown.data_ptr(), y.data_ptr(),
@@ -193,7 +187,7 @@ def moe_ffn_bwd_impl(dy, x, wr, wgu, wdown, top_k: int):
     need = _grouped_workspace(x2, wr, wgu, wdown, top_k, True)
     ws = _workspace(need, x.device) if need is not None and dy.dtype == x.dtype and dy.device == x.device else None
     if ws is not None:
-        dy2, x2, wr, wgu, wdown = (_packed(t) for t in (dy2, x2, wr, wgu, wdown))
+        dy2, x2, wr, wgu, wdown = (K.packed(t) for t in (dy2, x2, wr, wgu, wdown))
         dx, dwr, dwgu, dwdown = (torch.empty_like(t) for t in (x2, wr, wgu, wdown))
         E, _, F, _ = wgu.shape
         rc = _lib.load().mm_moe_bwd(dy2.data_ptr(), x2.data_ptr(), wr.data_ptr(), wgu.data_ptr(), wdown.data_ptr(),

@@ -101,3 +101,27 @@ def test_flash_attention_on_ragged_sequences(B, S, hkv, rep):
         assert fro(g[:, :, :, slot], gr[:, :, :, slot]) < 2e-2, (slot, fro(g[:, :, :, slot], gr[:, :, :, slot]))
     want = K.rope_(dqkv.clone().view(B * S, -1, D), *rope, backward=True, rot_per_group=rep + 1, group_size=rep + 2)
     assert fro(rotated.view(B * S, -1, D), want) < 2 ** -8
+
+
+@pytest.mark.parametrize("S", [96, 128, 200])
+def test_gradient_of_operands_that_are_views(S):
+    """Results and their gradients may start off a 16-byte boundary or be strided."""
+    from multimesh_jax_b200.ops import attention
+    B, hkv, rep, D = 2, 2, 2, 128
+    torch.manual_seed(S)
+    qkv = (torch.randn(B, S, hkv * (rep + 2), D, device="cuda") * 0.7).bfloat16()
+    dout = torch.randn(B, S, hkv * rep, D, device="cuda").bfloat16()
+    out, lse = attention.attention_fwd_packed(qkv, rep)
+    want = attention.attention_bwd_packed(dout, qkv, out, lse, rep)
+
+    def off(t):
+        flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+        flat[1:] = t.reshape(-1)
+        return flat[1:].view(t.shape)
+
+    strided = torch.stack([lse, lse], -1)[..., 0]
+    for d, o, l in ((off(dout), out, lse), (dout, off(out), lse), (dout, out, strided), (off(dout), off(out), off(lse))):
+        # the rows of dQ are summed with atomics, whose order is free: fp32 sums rounded to bf16
+        torch.testing.assert_close(attention.attention_bwd_packed(d, qkv, o, l, rep), want, rtol=2.0 ** -7, atol=1e-3)
+    assert torch.equal(attention.attention_bwd_packed(off(dout), qkv, off(out), strided, rep)[:, :, rep + 1::rep + 2],
+                       want[:, :, rep + 1::rep + 2])       # dV has no such sums

@@ -400,3 +400,15 @@ def test_sequence_parallel_tensor_parallel_step_matches_eager(pp, dp, tp, vocab)
     log = "\n".join(exe.plan.get("log", []))
     assert "collective folding" in log
     exe.shutdown()
+
+
+def test_attention_gradient_of_too_few_rows_is_refused():
+    from multimesh_jax_b200.ops import attention
+    qkv = torch.randn(2, 6, 4, 8)
+    out, lse = attention.attention_fwd_packed(qkv, 2)
+    dout = torch.randn_like(out)
+    want = attention.attention_bwd_packed(dout, qkv, out, lse, 2)
+    assert want.shape == qkv.shape
+    for bad in ((dout[:, :5], out, lse), (dout, out[:1], lse), (dout, out, lse[..., :5])):
+        with pytest.raises(ValueError, match="attention gradient"):
+            attention.attention_bwd_packed(bad[0], qkv, bad[1], bad[2], 2)
