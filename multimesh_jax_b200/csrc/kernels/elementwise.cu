@@ -435,11 +435,16 @@ __global__ void __launch_bounds__(CE_THREADS)
   const int64_t row = blockIdx.x;
   __nv_bfloat16* lr = logits + row * ld;
   const int64_t tgt = targets[row];
+  const int64_t local_t = tgt - vocab_start;
+  const bool has_t = tgt >= 0 && local_t >= 0 && local_t < V;
+  // read ahead of the barriers below: behind them the other threads write the gradient over the logits
+  const float tl = threadIdx.x == 0 && has_t ? __bfloat162float(lr[local_t]) : 0.f;
   const int nvec = V / 8;
   float mx, se;
   if (stats_in) {
     mx = stats_in[row * 2];
     se = stats_in[row * 2 + 1];
+    __syncthreads();
   } else {
     float m = -INFINITY, s = 0.f;
     for (int v = threadIdx.x; v < nvec; v += CE_THREADS) {
@@ -468,10 +473,7 @@ __global__ void __launch_bounds__(CE_THREADS)
     const float contrib = (m == -INFINITY) ? 0.f : s * __expf(m - mx);
     se = block_sum<CE_THREADS>(contrib, red);
   }
-  const int64_t local_t = tgt - vocab_start;
-  const bool has_t = tgt >= 0 && local_t >= 0 && local_t < V;
   if (threadIdx.x == 0) {
-    const float tl = has_t ? __bfloat162float(lr[local_t]) : 0.f;
     if (stats_out) {
       stats_out[row * 3] = mx;
       stats_out[row * 3 + 1] = se;

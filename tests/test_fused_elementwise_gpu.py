@@ -81,3 +81,13 @@ def test_scaling_in_place_by_one_and_by_another_factor():
             rc = _lib.load().mm_scale_bf16((y if out is y else x).data_ptr(), s.data_ptr(), out.data_ptr(), x.numel(),
                                            torch.cuda.current_stream().cuda_stream)
             assert rc == 0 and torch.equal(out, want)
+
+
+@pytest.mark.parametrize("rows,V", [(1, 8), (512, 1000), (8192, 32000), (1024, 128256)])
+def test_loss_does_not_depend_on_the_gradient_that_is_written_over_the_logits(rows, V):
+    logits, targets = _rand(rows, V), torch.randint(0, V, (rows,), device="cuda")
+    want = K.cross_entropy_fwd_bwd(logits, targets, 1.0, write_grad=False)
+    exact = torch.nn.functional.cross_entropy(logits[:512].double(), targets[:512], reduction="none")
+    torch.testing.assert_close(want[:512].double(), exact, rtol=1e-5, atol=1e-5)     # fp32 sums of V exponentials
+    for _ in range(4):
+        assert torch.equal(K.cross_entropy_fwd_bwd(logits.clone(), targets, 1.0, write_grad=True), want)
