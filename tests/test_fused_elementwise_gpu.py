@@ -60,6 +60,27 @@ def test_swiglu_widths(F):
     torch.testing.assert_close(K.swiglu_bwd(gu, dh).double(), want, rtol=2.0 ** -8 + 1e-4, atol=1e-5)
 
 
+# narrow rows, of which a block takes many, up to the width from which it takes one; counts that fill no block
+@pytest.mark.parametrize("F", [8, 24, 1016, 1024])
+@pytest.mark.parametrize("T,live", [(1, None), (301, None), (301, 0), (301, 7), (301, 400)])
+def test_swiglu_rows(F, T, live):
+    gu, dh = _rand(T, 2 * F), _rand(T, F)
+    g, u, d = gu[:, :F].double(), gu[:, F:].double(), dh.double()
+    s = torch.sigmoid(g)
+    rows = None if live is None else torch.tensor([live], device="cuda", dtype=torch.int32)
+    n = T if live is None else min(live, T)
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    count = rows.data_ptr() if rows is not None else None
+    h, dgu = torch.full((T, F), 7.0, device="cuda").bfloat16(), torch.full((T, 2 * F), 7.0, device="cuda").bfloat16()
+    assert lib.mm_swiglu_fwd_rows(gu.data_ptr(), h.data_ptr(), T, F, count, stream) == 0
+    assert lib.mm_swiglu_bwd_rows(gu.data_ptr(), dh.data_ptr(), dgu.data_ptr(), T, F, count, stream) == 0
+    # one bf16 rounding (2^-8 of the value at most) of a few 32-bit operations
+    torch.testing.assert_close(h[:n].double(), (g * s * u)[:n], rtol=2.0 ** -8 + 1e-5, atol=1e-6)
+    want = torch.cat([d * u * s * (1 + g * (1 - s)), d * g * s], 1)
+    torch.testing.assert_close(dgu[:n].double(), want[:n], rtol=2.0 ** -8 + 1e-4, atol=1e-5)
+    assert (h[n:] == 7.0).all() and (dgu[n:] == 7.0).all()
+
+
 @pytest.mark.parametrize("n", [4, 1024, 4 * 256 * 6 * 200 + 12])     # one vector; one block; more than one pass of the grid
 def test_adamw_walks_the_whole_buffer(n):
     torch.manual_seed(n)
