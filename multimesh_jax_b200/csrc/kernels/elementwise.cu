@@ -301,15 +301,24 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qk, const float* __restr
 }
 
 // The same rotation from `src` into another contiguous buffer, heads that are not rotated copied: one pass
-// where a copy and the in-place kernel take two. One block per token; bound by memory (with
-// the zero gradients of unused results left out, forward + backward of B1 S8192 32 / 8 heads 2.86 -> 2.81 ms).
+// where a copy and the in-place kernel take two. Bound by memory. One block per token, or - MANY - as many
+// whole tokens as fill its threads, where a token has fewer than half as many items as the block threads
+// (65536 tokens of 3 heads: 43 -> 23 us; copy and in-place rotation 34).
+template <bool MANY>
 __global__ void __launch_bounds__(256)
     rope_copy_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst, const float* __restrict__ cs,
-                     const float* __restrict__ sn, int S, int H, int Dh, int rot_per_group, int group_size) {
-  const int64_t t = blockIdx.x;
-  const int half = Dh / 2, per_head = half / 8;
+                     const float* __restrict__ sn, int64_t T, int S, int H, int Dh, int rot_per_group, int group_size) {
+  const int half = Dh / 2, per_head = half / 8, items = H * per_head;
+  int64_t t = blockIdx.x;
+  int first = threadIdx.x;
+  if (MANY) {
+    const int tokens = 256 / items, mine = first / items;
+    t = t * tokens + mine;
+    if (mine >= tokens || t >= T) return;
+    first -= mine * items;
+  }
   const int64_t pos = t % S;
-  for (int i = threadIdx.x; i < H * per_head; i += 256) {
+  for (int i = first; i < items; i += MANY ? items : 256) {
     const int h = i / per_head, c0 = (i - h * per_head) * 8;
     const int64_t at = (t * H + h) * Dh + c0;
     uint4 lo = *reinterpret_cast<const uint4*>(src + at), hi = *reinterpret_cast<const uint4*>(src + at + half);
@@ -781,9 +790,12 @@ int mm_rope_copy(const void* src, void* dst, const float* cos_t, const float* si
   if (Dh % 16 || ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15)) return -2;
   if (rot_per_group <= 0 || group_size <= 0) { rot_per_group = 1; group_size = 1; }
   if (T == 0 || H == 0) return 0;
-  rope_copy_kernel<<<static_cast<unsigned>(T), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(src),
-                                                                 static_cast<__nv_bfloat16*>(dst), cos_t, sin_t, S, H, Dh,
-                                                                 rot_per_group, group_size);
+  const int64_t items = static_cast<int64_t>(H) * (Dh / 16), tokens = items <= 128 ? 256 / items : 1;
+  const int64_t blocks = (T + tokens - 1) / tokens;
+  if (blocks > 0x7fffffff) return -2;
+  (tokens > 1 ? rope_copy_kernel<true> : rope_copy_kernel<false>)<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
+      static_cast<const __nv_bfloat16*>(src), static_cast<__nv_bfloat16*>(dst), cos_t, sin_t, T, S, H, Dh, rot_per_group,
+      group_size);
   MM_CUDA_TRY(cudaGetLastError());
   return 0;
 }

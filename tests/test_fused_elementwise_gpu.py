@@ -38,7 +38,8 @@ def test_add_rmsnorm_and_its_weight_gradient(D, rows):
 
 
 # a table shorter and longer than the token count; one head; groups with heads that are only copied
-@pytest.mark.parametrize("T,S,H,rot,group", [(1, 1, 1, 1, 1), (300, 300, 6, 2, 3), (256, 64, 12, 5, 6), (77, 1000, 3, 2, 3)])
+@pytest.mark.parametrize("T,S,H,rot,group", [(1, 1, 1, 1, 1), (300, 300, 6, 2, 3), (256, 64, 12, 5, 6), (77, 1000, 3, 2, 3),
+                                             (33, 33, 16, 3, 4), (31, 7, 17, 1, 1), (9, 9, 48, 5, 6)])
 def test_rotated_copy(T, S, H, rot, group):
     x = _rand(T, H, 128)
     cos, sin = K.rope_tables(S, 128, 1e4, "cuda")
