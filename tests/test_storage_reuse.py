@@ -283,3 +283,28 @@ def test_product_on_the_device(form):
             assert torch.equal(a.full_tensor(), b)
     assert any(v.startswith("native") for v in exe.native_report().values())
     exe.shutdown()
+
+
+def test_results_of_one_task_that_share_memory_are_left_to_each_other(monkeypatch):
+    """A task hands on a value twice, once as a view; the task that reads the first scales it, the next reads the second."""
+    torch.manual_seed(6)
+    args = (_b(8, 64), _b(64, 64), torch.tensor([0.5]).bfloat16())
+    mesh = mm.TaskMesh((1,), ("x",), [0])
+    first = mm.task(lambda x, w: (lambda y: (y, y.view(4, 2, 64)))(ops.linear(x, w)), name="first", mesh=mesh)
+    second = mm.task(lambda y, s, w: ops.linear(y * s, w), name="second", mesh=mesh)
+    third = mm.task(lambda v, w: ops.linear(v.view(8, 64), w), name="third", mesh=mesh)
+
+    def step(x, w, s):
+        y, v = first(x, w)
+        return second(y, s, w), third(v, w)
+
+    with mm.ignore_transforms():
+        want = step(*args)
+    mm.init(cpus=1)
+    exe = _compile(step, args)
+    assert len([op for op in exe.plan["ops"] if op["kind"] == "task"]) >= 3
+    assert not any(p.takes_over for p in exe.programs.values())
+    got, _ = _replay(exe, args, monkeypatch)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert all(torch.equal(a.full_tensor(), b) for a, b in zip(exe(*args), want))
+    exe.shutdown()
