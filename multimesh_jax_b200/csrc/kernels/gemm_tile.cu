@@ -366,10 +366,18 @@ int mm_gemm_tile_bf16(const void* A, int a_mn, int64_t lda, const void* B, int b
 //   512  512  1536   12.7      9.4      7.7         1500  1024 3072  20.4     15.2     18.7
 //   333  4096 4096   25.8     19.4     24.1         500   6144 4096  27.1     31.8     44.6
 //   333 28672 4096   89.8     97.9    123.4 (single CTA, 128x256 tiles: 83.0)
-// Forward + backward + accumulation of a d256 model (eight microbatches of 256 tokens): 8.22 -> 7.59 ms; of a
-// d1024 step on 500-token sequences 2.33 -> 2.25 ms.
+// Forward + backward + accumulation of a d256 model (eight microbatches of 256 tokens): 7.87 -> 7.59 ms; of a
+// d1024 step on 500-token sequences 2.33 -> 2.17 ms.
 // A K block of 64 takes 0.16 us on a 128x64 tile and 0.22 on 128x128 (both bound by what an SM takes in),
 // 0.30 .. 0.35 on a 256x256 pair and 0.40 on 128x256 (bound by the tensor cores); what an SM cannot run at once comes in rounds.
+// Every MB of operands that a K block brings in - on long, narrow problems nearly all of what the tiles read - costs
+// more, most where two small tiles share an SM. Without that term few columns and a long contraction took the small
+// tiles and up to twice the time (us, rule by rows alone | before | with the term):
+//   29216  280  9088     221   428   221 (pair)        14416   296  5400      79   126    79 (pair)
+//    4128 1072 18920     212   324   212 (pair)        10208   176  7400      60    91    60 (pair)
+// Of 1,860 random problems (8..32768 rows and columns, K 8..28672) that the terms were not fitted to, 1.2 % lose more
+// than a tenth against the rule by rows (before: 2.9 %), the worst of them 2 us of 8 on a size below one tile;
+// of 900 problems of model layers (widths 256..4096, 8..8192 tokens) none, and 2 % change their kernel.
 // pair_min_m: CTA pairs from this many rows on; 0: never.
 int mm_gemm_auto_bf16(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int out_mode,
                       int64_t ldc, int M, int N, int K, int pair_min_m, cudaStream_t stream) {
@@ -383,12 +391,14 @@ int mm_gemm_auto_bf16(const void* A, int a_mn, int64_t lda, const void* B, int b
   auto rounds = [](double ctas, int at_once) { return ceil(ctas / at_once); };
   const bool f32 = out_mode == OUT_F32 || out_mode == OUT_F32_ACC;
   const bool acc = out_mode == OUT_F32_ACC || out_mode == OUT_BF16_ACC;
-  double best = 6.0 + (acc ? 6.0 : f32 ? 2.0 : 0.0) + rounds(blocks(128, 256), sm) * kb * 0.40;
+  const double fresh = 0.035 * (static_cast<double>(M) + N) * (2e-6 * GT_BK);    // us per K block: its operands in MB
+  const double part = fmin(1.0, N / 256.0);                                     // of a persistent tile's columns
+  double best = 6.0 + (acc ? 6.0 : f32 ? 2.0 : 0.0) * part + rounds(blocks(128, 256), sm) * kb * (0.40 + fresh);
   bool pair = false;
   if (pair_min_m > 0 && M >= pair_min_m) {
     const double tiles = blocks(256, 256);
     const double full = tiles < sm / 2 ? tiles / (sm / 2) : 1.0;
-    const double t = 5.3 + (acc ? 4.2 : f32 ? 1.2 : 0.0) + rounds(tiles, sm / 2) * kb * (0.30 + 0.05 * full);
+    const double t = 5.3 + (acc ? 4.2 : f32 ? 1.2 : 0.0) * part + rounds(tiles, sm / 2) * kb * (0.30 + (0.05 + fresh) * full);
     if (t < best) { best = t; pair = true; }
   }
   int bn = 0, split = 0;
@@ -398,9 +408,9 @@ int mm_gemm_auto_bf16(const void* A, int a_mn, int64_t lda, const void* B, int b
       if (s > 1 && ctas > sm) break;      // a split pays only for SMs that would have stood idle
       double t = (n == 64 ? 3.4 : 4.0) + (acc ? (n == 64 ? 1.5 : 3.0) / s : 0.0) + (s > 1 ? 2.5 + 0.1 * s : 0.0);
       if (ctas <= sm)
-        t += k * (n == 64 ? 0.162 : 0.215);
+        t += k * (n == 64 ? 0.162 : 0.215 + fresh);
       else
-        t += rounds(ctas, 2 * sm) * (k * (n == 64 ? 0.31 : ctas <= 2 * sm ? 0.415 : 0.50) + 1.0);
+        t += rounds(ctas, 2 * sm) * (k * ((n == 64 ? 0.31 : ctas <= 2 * sm ? 0.415 : 0.50) + (ctas <= 2 * sm ? 4.6 : 2.9) * fresh) + 1.0);
       if (t < best) { best = t; bn = n; split = s; }
     }
   }
