@@ -280,6 +280,7 @@ class Executable:
                 local = sum(topology.is_local(shape["device_start"] + o) for o in range(shape["num_devices"]))
                 self._param_bytes += [n] * local
                 self._param_written += [sid in written] * local
+        self._plan_binding()
         # Debug aid for the compiler's buffer plan (MM_CHECK_LIFETIMES=1): stores that share a
         # physical buffer must never be alive at the same time. With the knob on, every tile
         # remembers which store wrote it last; a task or reshard that reads a store whose buffer
@@ -322,6 +323,17 @@ class Executable:
             kept |= {s for s, v in zip(op["inputs"], prog.inputs) if not plain or v not in clean[op["template"]]}
             kept |= set(op["outputs"])
         return {i for i, sid in enumerate(plan["param_stores"]) if sid >= 0 and sid not in kept}
+
+    def _plan_binding(self) -> None:
+        """What a call does with each argument: (argument, store, layout, its key, tiles must not share storage
+        with the caller's tensor, a task writes over tiles that were not donated)."""
+        self._binding = []
+        for i, sid in enumerate(self.plan["param_stores"]):
+            if sid >= 0:
+                want = self.plan["stores"][sid]["shape"]
+                donated = i in self.donated
+                self._binding.append((i, sid, want, want["key"], not donated and i not in self._shared_params,
+                                      not donated and i in self._written_params))
 
     def _copy_where_needed(self, bound: List[Tuple[int, int, Dict[int, torch.Tensor]]]) -> None:
         """Replaces tiles of the step's arguments, given as (argument, store, tiles per device), by copies:
@@ -653,19 +665,16 @@ class Executable:
             self._created = True
         # parameter stores
         bound: List[Tuple[int, int, Dict[int, torch.Tensor]]] = []
-        for i, sid in enumerate(plan["param_stores"]):
-            if sid < 0:
-                continue
-            want = plan["stores"][sid]["shape"]
+        for i, sid, want, key, private, written in self._binding:
             a = tensors[i]
             if isinstance(a, ShardedTensor):
-                if a.sharding["key"] != want["key"]:
+                if a.sharding["key"] != key:
                     a = shard_tensor(a.full_tensor(), want, topo)
                 new_tiles = a.local_tiles()
-                if i in self._written_params and i not in self.donated:
+                if written:
                     new_tiles = {d_: t.clone() for d_, t in new_tiles.items()}
             else:
-                new_tiles = shard_tensor(a, want, topo, private=i not in self.donated and i not in self._shared_params).local_tiles()
+                new_tiles = shard_tensor(a, want, topo, private=private).local_tiles()
             bound.append((i, sid, new_tiles))
         self._copy_where_needed(bound)
         for _, sid, new_tiles in bound:

@@ -76,6 +76,7 @@ def test_tiles_of_arguments_start_on_vector_boundaries(donate):
     exe, args = _loss_step("cpu", train=donate)
     exe._shared_params = set(range(len(exe.plan["param_stores"])))      # as on a device: nothing is copied for privacy
     exe.donated = set(exe._shared_params) if donate else set()
+    exe._plan_binding()
     want = exe(*pytree.tree_map(torch.clone, args))[0].full_tensor()
     odd = pytree.tree_map(_offset_view, args)
     even = pytree.tree_map(torch.clone, args)
@@ -136,6 +137,7 @@ def test_one_tensor_passed_as_a_written_and_as_a_read_argument():
         exe = mm.compile_function(step, (p, *[flat[:64]] * 3, g, t, flat[:64]), num_devices=1, backend="cpu",
                                   donate_argnums=(0, 1, 2, 3))
     exe._shared_params = {4, 5, 6}      # as on a device
+    exe._plan_binding()
     # (master, m, v, ref): apart; ref is the master; ref lies across two of them; both moments and ref are one tensor
     for spans in ((0, 64, 128, None), (0, 64, 128, 0), (0, 64, 128, 32), (0, 64, 64, 64), (0, 0, 0, 0)):
         memory = flat.clone()
