@@ -670,7 +670,9 @@ class Executable:
             if isinstance(a, ShardedTensor):
                 if a.sharding["key"] != key:
                     a = shard_tensor(a.full_tensor(), want, topo)
-                new_tiles = a.local_tiles()
+                if a._waiter is not None:
+                    a.wait()
+                new_tiles = dict(a._tiles)
                 if written:
                     new_tiles = {d_: t.clone() for d_, t in new_tiles.items()}
             else:
