@@ -21,35 +21,29 @@
 // others = softmax / epilogue (TMEM lane quarter = warp % 4; four warps forward, eight - two per
 // quarter, splitting the columns - and four for dQ backward). The backward TMA warp also brings the step's
 // log-sum-exp and delta rows into shared memory with the step's Q / dO tiles, two steps ahead of
-// their use: as global loads of the compute warps they queued in the load/store unit behind the
-// 32 dQ reductions every thread issues per step. All waits are bounded.
+// their use: as global loads they queued in the load/store unit behind the dQ reductions. All waits are bounded.
 //
 // Ragged sequences run on the same tiles: TMA zero-fills what lies behind the sequence, causality
 // masks it for every row inside, and rows outside are not stored. B4 H16 S1000 forward + backward
-// takes 0.248 ms against 0.462 ms through the library kernels this replaced. The backward pass has
+// takes 0.197 ms against 0.460 ms through the library kernels this replaced. The backward pass has
 // one kernel ahead of it (row statistics and the zeroed dQ accumulator) and one behind it (dQ to
 // bf16); both gradients that passed through the rotary embedding are rotated back where they are
 // stored, which saves a read-modify-write pass (B1 S8192 32 / 8 heads, whole call: 3.138 -> 3.088 ms).
 //
-// Measured on the backward call (B4 H32 S2048, one GPU, alternating runs; 0.816 ms before): a
-// three-stage Q / dO ring 0.793 ms, ex2.approx instead of exp2f 0.780 ms, the staged rows on top
-// of the ring 0.700 ms (all kept; forward 0.252 -> 0.233 ms with ex2.approx). The same staging
-// with a two-stage ring was slower (0.940 ms: the rows arrived with the tiles, one step ahead,
-// and the compute warps waited for them). Also not kept: sixteen compute warps of 16 columns
-// (3 % slower before the staging, 0.6 % faster after it), dQ through shared memory and cp.reduce.async.bulk (0.92 ms; 0.86 ms against 0.70
-// with a reducer warp of its own), dQ reductions
-// interleaved with the next step's exponentials (0.86 ms). A cycle-stamped trace of one CTA
-// before these changes: 5,200 cycles per 64-query step, the eight compute warps busy for 4,500
-// of them (exponentials 1,280, dS 970, the dQ reductions 1,320), the MMA lane issuing its 32
-// small (N = 64) instructions in 2,300.
-// The MMA lane's share fell when it became an elected lane with its descriptors made once (see elect_one
-// in ptx.cuh): whole call of forward + backward, B1 S8192 32 / 8 heads 3.04 -> 2.85 ms, B4 H16 S1000
-// 0.249 -> 0.233 ms.
-// Forward: the exponentials now run before the wait for the previous product, and the maximum and the sum
-// are four chains each; the scale is part of the exponent's multiply-add (same call 2.83 -> 2.77 ms).
-// Backward: dQ leaves TMEM through four warps of their own, which turn the tile around in shared memory and
-// add 512 bytes per instruction (2.76 -> 2.70 ms, the ragged case 0.227 -> 0.206). The same warps with one
-// float per lane were slower (3.06): four warps issue 256 reductions a step later than eight do.
+// What the structure rests on, each measured against the other form at the time (ms; the call is forward +
+// backward unless it says otherwise):
+//   three-stage Q / dO ring, row statistics by TMA      backward B4 H32 S2048  0.816 -> 0.700 with ex2.approx
+//     with a two-stage ring (rows one step ahead)       0.940
+//   elected issue with ready descriptors (ptx.cuh)      B1 S8192 32 / 8 heads  3.04 -> 2.85, B4 H16 S1000 0.249 -> 0.233
+//   forward: exponentials ahead of the wait for the previous product, maximum and sum as four chains each, the
+//     scale inside the exponent's multiply-add          B1 S8192 32 / 8 heads  2.83 -> 2.77
+//   backward: dQ through four warps of its own, whole rows per reduction
+//                                                       B1 S8192 32 / 8 heads  2.76 -> 2.70, B4 H16 S1000 0.227 -> 0.206
+//     the same warps with one float per lane            B1 S8192 32 / 8 heads  3.06
+//     dQ through shared memory and cp.reduce.async.bulk backward B4 H32 S2048  0.86 (against 0.70)
+// What bounds it: backward, the chain of one 64-query step (exponentials, dS, shared-memory stores, two waits)
+// through one P^T / dS^T buffer each; forward, the exponentials. Blocks of all lengths of one head start
+// before those of the next, so the last head's longest blocks end alone.
 #include <math.h>
 
 #include "host_common.h"
@@ -111,7 +105,7 @@ __global__ void __launch_bounds__(FA_THREADS, 2)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  const int q_blk = gridDim.x - 1 - blockIdx.x;  // longest rows first
+  const int q_blk = gridDim.x - 1 - blockIdx.x;  // longest rows first, within one head: blocks start with x fastest
   const int hq = blockIdx.y, b = blockIdx.z;
   const int g = hq / p.rep, r = hq - g * p.rep;
   const int hp_q = g * (p.rep + 2) + r, hp_k = g * (p.rep + 2) + p.rep, hp_v = hp_k + 1;
@@ -387,7 +381,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
   float* sDQ = sRow + FB_QST * FB_ROWBLK;                         // [64 query rows][128]
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  const int jb = blockIdx.x;  // key block; block 0 has the most query blocks and starts first
+  const int jb = blockIdx.x;  // key block; block 0 has the most query blocks and starts first within its head
   const int g = blockIdx.y, b = blockIdx.z;
   const int Hq = p.Hkv * p.rep;
   const int hp_k = g * (p.rep + 2) + p.rep, hp_v = hp_k + 1;

@@ -624,8 +624,8 @@ __global__ void adamw_kernel(float* __restrict__ master, __nv_bfloat16* __restri
                              float beta2, float eps, float wd, float bc1, float bc2,
                              float grad_scale, const int64_t* __restrict__ step_dev) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  // Memory bound (28 bytes per element) only while the arithmetic stays short: the two powers of the bias
-  // correction are computed by one thread per block, under the loads of the others (267 -> 232 us per call,
+  // Memory bound (30 bytes per element) only while the arithmetic stays short: the two powers of the bias
+  // correction are computed by two threads per block, under the loads of the others (267 -> 232 us per call,
   // the mean of a step of two 7B layers). A few blocks per SM that walk the buffer and compute them once per
   // thread were slower: 307 us.
   __shared__ float bc[2];
