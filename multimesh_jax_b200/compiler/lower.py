@@ -92,6 +92,7 @@ class TemplateProgram:
         self.device_start = template["device_start"]
         self._last_use = last_use
         self.fused_acc: Dict[int, bool] = {}
+        self.storage: Optional[StorageUse] = None
         # (instruction index, operand id) of the operands that an operator may write its result over
         self.takes_over: set = set()
         # the inputs that some operator of the task may write over
@@ -225,14 +226,14 @@ class StorageUse:
         self.root: Dict[int, int] = {v: v for v in inputs}
         self.partial: set = set()
         self.inputs = set(inputs)
-        self.instrs = instrs
-        last: Dict[int, int] = {}
+        self.reads = [_reads(ins) for ins in instrs]
+        self.last: Dict[int, int] = {}              # value -> last instruction that reads it
         for idx, ins in enumerate(instrs):
-            for v in _reads(ins):
-                last[v] = idx
+            for v in self.reads[idx]:
+                self.last[v] = idx
             src, whole = None, True
             if ins.kind in (0, 1, 3, 4, 5, 6):
-                src, whole = _storage_source(g.node(ins.node_id)["op"], _reads(ins))
+                src, whole = _storage_source(g.node(ins.node_id)["op"], self.reads[idx])
             for o in ins.outs or ():
                 self.root[o] = o if src is None else self.root.get(src, src)
                 if src is not None and (not whole or src in self.partial):
@@ -240,7 +241,7 @@ class StorageUse:
         self.needed_until: Dict[int, int] = {}      # root -> last instruction that reads any value in its memory
         kept = set(outputs)
         for v, r in self.root.items():
-            end = len(instrs) if v in kept else last.get(v, -1)
+            end = len(instrs) if v in kept else self.last.get(v, -1)
             self.needed_until[r] = max(self.needed_until.get(r, -1), end)
 
     def dies_with(self, idx: int, vid: int, overwritable: set) -> bool:
@@ -248,11 +249,11 @@ class StorageUse:
         operand, so the instruction may write a result over it. Memory of a task input qualifies only
         when it is in ``overwritable``."""
         root = self.root.get(vid, vid)
-        if vid in self.partial or self.needed_until.get(root, len(self.instrs)) > idx:
+        if vid in self.partial or self.needed_until.get(root, len(self.reads)) > idx:
             return False
         if root in self.inputs and root not in overwritable:
             return False
-        return sum(self.root.get(v, v) == root for v in _reads(self.instrs[idx])) == 1
+        return sum(self.root.get(v, v) == root for v in self.reads[idx]) == 1
 
 
 def overwritable_inputs(cap: Captured, plan: dict) -> Dict[int, Tuple[set, set, set]]:
@@ -571,25 +572,21 @@ def build_program(cap: Captured, plan: dict, template: dict, fast_ops: Optional[
             prod.extra = (pos, acc_dtype)
             fused_acc[pos] = True
     # liveness inside the program
-    last: Dict[int, int] = {}
+    use = StorageUse(g, instrs, template["inputs"], template["outputs"])
     keep = set(template["outputs"])
-    for idx, ins in enumerate(instrs):
-        for v in _reads(ins):
-            last[v] = idx
     # An operator may write its result over an operand when nothing needs the operand's memory afterwards:
     # no value of this task that lies in it, no other reader of the store behind a task input. The native
     # program asks the same set; here the operators with a variant that does so fall back to the plain
     # form (AdamW: per operand) where the rule refuses.
     from ..ops.mm_ops import MAY_WRITE_OVER
     temps, sole_args, last_args = (overwritable or overwritable_inputs(cap, plan)).get(template["id"], (set(), set(), set()))
-    use = StorageUse(g, instrs, template["inputs"], template["outputs"])
     takes_over, written_inputs = set(), set()
     plain_of = {id(ins): plain for ins, plain, _ in fast_variants}
     for idx, ins in enumerate(instrs):
         opname = g.node(ins.node_id)["op"] if ins.kind == 0 else None
         if opname not in MAY_WRITE_OVER:
             continue
-        ids = _tensor_ids_in_order(ins.args, ins.kwargs)
+        ids = use.reads[idx]
         operands = [ids[pos] for pos, _ in MAY_WRITE_OVER[opname] if pos < len(ids)]
         update = opname == "mm_ops.adamw.default"      # the one operator that may take over step arguments
         taken = {v for v in operands if use.dies_with(idx, v, temps | sole_args if update else temps)}
@@ -600,12 +597,12 @@ def build_program(cap: Captured, plan: dict, template: dict, fast_ops: Optional[
         if id(ins) in plain_of and not all(dead):
             ins.fn = functools.partial(ins.fn, overwrite=tuple(dead)) if update else plain_of[id(ins)]
     last_use: Dict[int, List[int]] = {}
-    for v, idx in last.items():
+    for v, idx in use.last.items():
         if v not in keep:
             last_use.setdefault(idx, []).append(v)
     prog = TemplateProgram(template, instrs, list(template["inputs"]), list(template["outputs"]), last_use)
     prog.fused_acc = fused_acc
-    prog.takes_over, prog.written_inputs = takes_over, written_inputs
+    prog.storage, prog.takes_over, prog.written_inputs = use, takes_over, written_inputs
     return prog
 
 

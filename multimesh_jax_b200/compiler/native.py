@@ -38,7 +38,7 @@ from ..ops import _lib
 from ..ops import attention as _attention  # noqa: F401  (declares the attention entry points)
 from .capture import DTYPE_FROM_NAME
 from ..ops.mm_ops import MAY_WRITE_OVER
-from .lower import Instr, StorageUse, TemplateProgram, _reads, _tensor_ids_in_order, _V
+from .lower import Instr, TemplateProgram, _tensor_ids_in_order, _V
 
 ALIGN = 256
 
@@ -660,12 +660,12 @@ def inputs_left_alone(cap, prog: TemplateProgram) -> set:
     """The inputs of ``prog`` whose storage the task only reads: no operator may write over them, and
     neither they nor a view of them is among the task's outputs. An operator this module does not
     know counts as one that might do either."""
-    root = StorageUse(cap.graph, prog.instrs, prog.inputs, prog.outputs).root
+    root = prog.storage.root
     touched = set(prog.written_inputs) | {root.get(v, v) for v in prog.outputs}
-    for ins in prog.instrs:
+    for ins, reads in zip(prog.instrs, prog.storage.reads):
         op = cap.graph.node(ins.node_id)["op"] if ins.kind in (0, 6) else None
         if ins.kind not in (1, 2, 3) and op not in EMITTERS:
-            touched |= {root.get(v, v) for v in _reads(ins)}
+            touched |= {root.get(v, v) for v in reads}
     return set(prog.inputs) - touched
 
 
@@ -706,7 +706,7 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
         b.env[v] = Sym(i, 0, shape, DTYPE_FROM_NAME[val["dtype"]])
     # Operands that take a result: the program's own decision, less the inputs that must stay.
     protected = {prog.inputs[i] for i in protected_inputs}
-    root_of = StorageUse(g, prog.instrs, prog.inputs, prog.outputs).root
+    root_of = prog.storage.root
     takes_over = {(idx, v) for idx, v in prog.takes_over if root_of.get(v, v) not in protected}
     # Values whose storage a task output ends up naming - directly, through view-like operators
     # (autograd hands saved tensors on as detached aliases) or because an operator writes its
@@ -733,8 +733,8 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
                     b.reaches_ext.setdefault(alias_parent[o], b.reaches_ext[o])
     # Weight gradients of the norms that nothing but an accumulated output reads: value -> output position
     readers: Dict[int, int] = {}
-    for ins in prog.instrs:
-        for v in _reads_of(ins):
+    for reads in prog.storage.reads:
+        for v in reads:
             readers[v] = readers.get(v, 0) + 1
     b.sole_accumulator = {}
     for k, v in enumerate(prog.outputs):
@@ -841,12 +841,6 @@ def build_native(cap, plan: dict, template: dict, prog: TemplateProgram, accumul
     b.np.out_block_bytes = sum(b.out_chunks)
     b.np.scratch_bytes = b.scratch.peak
     return b.np
-
-
-def _reads_of(ins: Instr) -> List[int]:
-    if ins.kind in (0, 6):
-        return _tensor_ids_in_order(ins.args, ins.kwargs)
-    return [ins.args] if isinstance(ins.args, int) else []
 
 
 def plan_store_dtype(plan: dict, template: dict, out_pos: int) -> str:
