@@ -485,11 +485,22 @@ class Executable:
             scratch = max([scratch] + [n.scratch_bytes for n in built.values()])
         self.native_scratch_bytes = scratch
         if self._native:
-            for d in self.topology.local_devices:
+            self._reserve_scratch(scratch)
+
+    def _reserve_scratch(self, scratch: int) -> None:
+        """The scratch tile of the native programs, sized for the largest. Where a device cannot supply it,
+        with nothing left in the allocator's cache either, every task keeps its interpreted program."""
+        for d in self.topology.local_devices:
+            base = self.context.reserve_scratch(d, max(scratch, 1 << 20))
+            if not base:
+                torch.cuda.empty_cache()
                 base = self.context.reserve_scratch(d, max(scratch, 1 << 20))
-                if not base:
-                    raise MemoryError(f"cannot reserve {scratch} bytes of task scratch on device {d}")
-                self._scratch_base[d] = base
+            if not base:
+                for tid, _ in self._native:
+                    self._native_why[tid] = f"{scratch >> 20} MiB of task scratch could not be reserved on device {d}"
+                self._native.clear()
+                return
+            self._scratch_base[d] = base
 
     def native_report(self) -> Dict[str, str]:
         """Per template: ``native (<n> kernel calls)`` or why it keeps the interpreted program."""

@@ -89,3 +89,14 @@ def test_fresh_outputs_are_carved_from_bounded_chunks(monkeypatch):
         assert total <= (256 << 10) or len(sizes.get(chunk, ())) <= 1
     assert split.num_calls == whole.num_calls
     exe.shutdown()
+
+
+def test_tasks_are_interpreted_when_the_scratch_tile_cannot_be_reserved():
+    from types import SimpleNamespace
+    from multimesh_jax_b200.runtime.executable import Executable
+    for answers, native in (([64], True), ([0, 64], True), ([0, 0], False)):
+        exe = SimpleNamespace(topology=SimpleNamespace(local_devices=[0]), _native={(3, False): "a", (3, True): "b"}, _native_why={},
+                              _scratch_base={}, context=SimpleNamespace(reserve_scratch=lambda d, n: answers.pop(0)))
+        Executable._reserve_scratch(exe, 5 << 20)
+        assert answers == [] and bool(exe._native) == native and exe._scratch_base == ({0: 64} if native else {})
+        assert native or exe._native_why == {3: "5 MiB of task scratch could not be reserved on device 0"}
