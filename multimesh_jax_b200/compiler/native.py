@@ -175,14 +175,15 @@ def _linear_bwd(first, second):
 
 
 def _cross_entropy_to(first, second):
-    """A copy of the logits and the loss that turns the copy into its gradient: one pass from one to the other."""
+    """A copy of the logits and the loss that turns the copy into its gradient: one pass from one to the other. It reads
+    the logits while it writes: they may not be where the gradient goes, nor, dead once they are copied, the losses."""
     (n1, copy), (n2, ce) = first, second
     if n1 != "mm_memcpy_d2d" or n2 != "mm_cross_entropy":
         return None
     grad, logits, nbytes, _ = copy
     buf, targets, loss, stats_out, stats_in, rows, V, ld, start, scale, write, _ = ce
     if (not _same(grad, buf) or nbytes != buf.nbytes or buf.numel != rows * V or (stats_out, stats_in, ld, start, write) != (None, None, V, 0, 1)
-            or not _disjoint([grad], [logits])):
+            or not _disjoint([grad, loss], [logits])):
         return None
     return "mm_cross_entropy_to", (logits, grad, targets, loss, rows, V, scale, STREAM)
 

@@ -165,6 +165,42 @@ def test_a_copy_of_the_logits_for_their_gradient_is_one_pass():
     assert len(merge_calls([copy, (ce[0], ce[1][:10] + (0, STREAM))])) == 2                  # no gradient
 
 
+def test_the_losses_do_not_go_over_logits_that_the_same_pass_reads(monkeypatch):
+    """Logits that are copied by the program itself die with the copy, so the losses of the rows take their memory:
+    fine behind the copy, not in one pass that reads them."""
+    from multimesh_jax_b200.compiler import native
+    logits, grad, tok = _sym(0, 0, 4, 16), _sym(1, 0, 4, 16), _sym(2, 0, 4, dtype=torch.int64)
+    for at, calls in ((0, 2), (112, 2), (128, 1)):
+        loss = _sym(0, at, 4, dtype=torch.float32)
+        copy = ("mm_memcpy_d2d", (grad, logits, 128, native.STREAM))
+        ce = ("mm_cross_entropy", (grad, tok, loss, None, None, 4, 16, 16, 0, 0.5, 1, native.STREAM))
+        assert len(native.merge_calls([copy, ce])) == calls
+
+    seen = []
+    add = native._Builder._add_call
+    monkeypatch.setattr(native._Builder, "_add_call", lambda self, name, a: (seen.append((name, a)), add(self, name, a))[1])
+    ops = torch.ops.mm_ops
+    x, w, t = torch.randn(64, 64).bfloat16(), torch.randn(512, 64).bfloat16(), torch.randint(0, 512, (64,))
+
+    def step(x, w, t):
+        z = ops.linear(x, w).to(torch.bfloat16, copy=True)
+        return tuple(ops.cross_entropy(z, t, 0.125))
+
+    with mm.enable_fast_path(False):
+        exe = mm.compile_function(step, (x, w, t), num_devices=1, backend="cpu")
+    for op in exe.plan["ops"]:
+        if op["kind"] == "task":
+            tm = exe.plan["templates"][op["template"]]
+            build_native(exe.cap, exe.plan, tm, exe.programs[tm["id"]], tuple(int(m > 0) for m in op["accumulate"]), False)
+    exe.shutdown()
+    (copied,) = [a for n, a in seen if n == "mm_memcpy_d2d"]
+    (ce,) = [a for n, a in seen if n == "mm_cross_entropy"]
+    assert not native._disjoint([ce[2]], [copied[1]])       # the case in question: losses over the copied logits
+    for name, a in seen:
+        if name == "mm_cross_entropy_to":
+            assert native._disjoint([a[1], a[3]], [a[0]])
+
+
 def test_the_gradient_of_a_loss_is_not_written_when_nothing_reads_it(monkeypatch):
     from multimesh_jax_b200.compiler import native
     seen = []
