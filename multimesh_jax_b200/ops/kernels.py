@@ -422,7 +422,8 @@ def cross_entropy_fwd_bwd(logits: torch.Tensor, targets: torch.Tensor, grad_scal
 def cross_entropy_to(logits: torch.Tensor, targets: torch.Tensor, grad_scale: float) -> Tuple[torch.Tensor, torch.Tensor]:
     """(per-row loss, gradient in a buffer of its own) of :func:`cross_entropy_fwd_bwd`; the logits stay."""
     rows, V = logits.shape
-    if logits.is_cuda and logits.dtype == bf16 and logits.is_contiguous() and V % 8 == 0:
+    # the kernel loads 16 bytes at a time; a copy starts on them
+    if logits.is_cuda and logits.dtype == bf16 and logits.is_contiguous() and V % 8 == 0 and logits.data_ptr() % 16 == 0:
         grad = torch.empty_like(logits)
         loss = torch.empty(rows, dtype=torch.float32, device=logits.device)
         rc = _lib.load().mm_cross_entropy_to(logits.data_ptr(), grad.data_ptr(), targets.data_ptr(), loss.data_ptr(), rows, V,

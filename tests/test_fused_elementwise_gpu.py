@@ -167,3 +167,14 @@ def test_loss_gradient_into_another_buffer(rows, V):
     assert torch.equal(logits, before)
     want = before.clone()
     assert torch.equal(K.cross_entropy_fwd_bwd(want, targets, 0.5), loss) and torch.equal(want, grad)
+
+
+@pytest.mark.parametrize("offset", [1, 4, 8])
+def test_loss_gradient_of_logits_that_start_off_16_bytes(offset):
+    rows, V = 70, 2056
+    flat, targets = _rand(rows * V + 8), torch.randint(0, V, (rows,), device="cuda")
+    logits = flat[offset:offset + rows * V].view(rows, V)
+    assert logits.is_contiguous() and logits.data_ptr() % 16 == offset * 2 % 16
+    loss, grad = torch.ops.mm_ops.cross_entropy(logits, targets, 0.5)
+    want = logits.clone()
+    assert torch.equal(K.cross_entropy_fwd_bwd(want, targets, 0.5).sum() * 0.5, loss) and torch.equal(want, grad)
