@@ -444,9 +444,6 @@ __device__ __forceinline__ void staged8(const float* stage, int row, int col, ui
   hi[0] = d.x; hi[1] = d.y; hi[2] = d.z; hi[3] = d.w; hi[4] = e.x; hi[5] = e.y; hi[6] = e.z; hi[7] = e.w;
 }
 
-__device__ __forceinline__ void fb_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float4 fb_ld_cluster(uint32_t addr, uint32_t rank) {
   uint32_t a;
   float4 v;
@@ -841,7 +838,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
   }
 
   if (p.split > 1) {
-    fb_cluster_sync();
+    cluster_sync();
     if (warp >= 4 && warp < 12) {
       const int rows = FB_BLK / p.split;
       for (int u = static_cast<int>(threadIdx.x) - 128; u < 2 * rows * 8; u += 256) {
@@ -869,8 +866,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
         store_grad8(p, b, hp_k + which, pos, col, lo, hi);
       }
     }
-    __syncwarp();
-    fb_cluster_sync();   // nobody leaves while a partner may still read its sums
+    cluster_sync();   // nobody leaves while a partner may still read its sums
   }
 
   tc_fence_before();

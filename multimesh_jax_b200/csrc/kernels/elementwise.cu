@@ -348,7 +348,7 @@ __global__ void __cluster_dims__(RC_CTAS, 1, 1) __launch_bounds__(32 * WARPS)
     for (int k = 0; k < WARPS; ++k) t += part[k][j];
     part[0][j] = t;
   }
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_sync();
   const int share = nvec;          // D / 8 columns for each of the eight CTAs
   static_assert(RC_CTAS == 8, "a CTA finishes an eighth of the columns");
   if (static_cast<int>(threadIdx.x) < share) {
@@ -366,7 +366,7 @@ __global__ void __cluster_dims__(RC_CTAS, 1, 1) __launch_bounds__(32 * WARPS)
     if (ROUND) t = __bfloat162float(__float2bfloat16(t));
     dw[j] = accumulate ? static_cast<OUT>(static_cast<float>(dw[j]) + t) : static_cast<OUT>(t);
   }
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");   // partners may still read
+  cluster_sync();   // partners may still read
 }
 
 // --------------------------------------------------------------------- RoPE

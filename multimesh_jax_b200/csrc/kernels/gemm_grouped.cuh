@@ -86,8 +86,7 @@ struct GroupedSmem {
     for (int i = threadIdx.x; i < GG_PLAN; i += blockDim.x) plan[i] = plan_dev[i];
     tc_fence_before();
     __syncthreads();
-    cluster_arrive();
-    cluster_wait();
+    cluster_sync();
     tc_fence_after();
     return *tmem_slot;
   }
@@ -96,8 +95,7 @@ struct GroupedSmem {
   __device__ void end(uint32_t tmem_base) {
     tc_fence_before();
     __syncthreads();
-    cluster_arrive();
-    cluster_wait();
+    cluster_sync();
     if (warp_index() == 1) {
       tc_fence_after();
       tmem_dealloc_pair(tmem_base, 512);

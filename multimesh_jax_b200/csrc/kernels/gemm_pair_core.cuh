@@ -44,12 +44,6 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_arrive() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // shared::cluster address of `p` (an address in this CTA's shared memory) inside CTA `rank`
 __device__ __forceinline__ uint32_t mapa_u32(const void* p, uint32_t rank) {
   uint32_t out;
@@ -151,8 +145,7 @@ __global__ void __launch_bounds__(G2_THREADS + 32 * Hook::kAuxWarps, 1)
   }
   tc_fence_before();
   __syncthreads();
-  cluster_arrive();
-  cluster_wait();
+  cluster_sync();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -255,8 +248,7 @@ __global__ void __launch_bounds__(G2_THREADS + 32 * Hook::kAuxWarps, 1)
   // or run MMAs on its tensor memory
   tc_fence_before();
   __syncthreads();
-  cluster_arrive();
-  cluster_wait();
+  cluster_sync();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, 512);

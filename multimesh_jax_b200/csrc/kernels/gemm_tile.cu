@@ -38,9 +38,6 @@ __device__ __forceinline__ uint32_t gt_cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void gt_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float4 gt_ld_cluster(uint32_t addr, uint32_t rank) {
   uint32_t a;
   float4 v;
@@ -232,7 +229,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmA, const CUt
   } else {
     // CTA `rank` sums and stores rows [rank, rank + 1) * 128 / split of the tile
     const int good = __syncthreads_and(ok);
-    gt_cluster_sync();
+    cluster_sync();
     if (good) {
       const int rows = GT_BM / split, wrows = rows / 4;
       for (int r0 = 0; r0 < wrows; r0 += RPI) {
@@ -248,7 +245,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmA, const CUt
         if (m0 + r < M && n0 + col < N) gt_store8<OUT>(C, ldc, m0 + r, n0 + col, N, a, b, vec_ok);
       }
     }
-    gt_cluster_sync();                // nobody leaves while a partner may still read its tile
+    cluster_sync();                // nobody leaves while a partner may still read its tile
   }
   tc_fence_before();
   __syncthreads();

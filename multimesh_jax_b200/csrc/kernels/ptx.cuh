@@ -86,6 +86,13 @@ __device__ __forceinline__ bool elect_one() {
 // Index of this thread's warp in its block, known to be the same in every lane.
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x) >> 5, 0); }
 
+// Barrier over all threads of a cluster; what they wrote before it is visible behind it. The aligned instructions
+// want every warp whole, and callers come out of loops and branches that lanes leave one by one.
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
