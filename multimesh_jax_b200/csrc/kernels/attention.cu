@@ -1036,7 +1036,7 @@ int mm_flash_attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int 
   p.order = block_order(static_cast<int64_t>(B) * Hkv * rep, static_cast<int64_t>(S) * FA_D * 4 / rep + 1, nblk, 2 * ds->sm_count);
   const unsigned grid = static_cast<unsigned>(p.order.heads) * nblk;
   flash_fwd_kernel<<<grid, FA_THREADS, FA_FWD_SMEM, stream>>>(tmQ, tmKV, p, ds->status);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -1117,7 +1117,7 @@ int mm_flash_attn_bwd(const void* qkv, const void* out, const void* dout, const 
   cfg.numAttrs = p.split > 1 ? 1 : 0;
   MM_CUDA_TRY(cudaLaunchKernelEx(&cfg, direct ? flash_bwd_kernel<true> : flash_bwd_kernel<false>, tmQKV, tmDO, p, ds->status));
   if (!direct) flash_dq_store_kernel<<<static_cast<unsigned>(tiles * 4), 256, 0, stream>>>(p);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(direct ? 1 : 3);
   return 0;
 }
 

@@ -843,7 +843,7 @@ static int launch_rmsnorm_fwd(const void* x, const void* delta, void* xn, const 
   else if (D <= 8192) MM_RN_FWD(256, 4);
   else MM_RN_FWD(512, 4);
 #undef MM_RN_FWD
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int64_t rows, int D,
@@ -886,7 +886,7 @@ static int rmsnorm_bwd(const void* x, const void* w, const void* dy, const float
     const int n = static_cast<int>(rows);
     if (D <= 256) rmsnorm_bwd_cluster_kernel<1, 16, OUT, ROUND><<<RC_CTAS, 512, 0, stream>>>(xb, wb, gb, rstd, db, dw_out, n, D, accumulate_dw, add_to_dx);
     else rmsnorm_bwd_cluster_kernel<2, 16, OUT, ROUND><<<RC_CTAS, 512, 0, stream>>>(xb, wb, gb, rstd, db, dw_out, n, D, accumulate_dw, add_to_dx);
-    MM_CUDA_TRY(cudaGetLastError());
+    MM_LAUNCHED(1);
     return 0;
   }
   const int parts = mm_rmsnorm_bwd_parts(rows);
@@ -901,10 +901,10 @@ static int rmsnorm_bwd(const void* x, const void* w, const void* dy, const float
   else if (D <= 8192) MM_RN_BWD(512, 2);
   else MM_RN_BWD(512, 4);
 #undef MM_RN_BWD
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   if (parts > 64) colsum_partials_kernel<OUT, ROUND, 32><<<(D + 31) / 32, 1024, 0, stream>>>(scratch, dw_out, parts, D, accumulate_dw);
   else colsum_partials_kernel<OUT, ROUND, 8><<<(D + 31) / 32, 256, 0, stream>>>(scratch, dw_out, parts, D, accumulate_dw);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -938,7 +938,7 @@ int mm_rope(void* qk, const float* cos_t, const float* sin_t, int64_t T, int S, 
                                                          sin_t, T, S, H, Dh, stride_t,
                                                          backward ? -1.f : 1.f, rot_per_group,
                                                          group_size);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -954,7 +954,7 @@ int mm_rope_copy(const void* src, void* dst, const float* cos_t, const float* si
   (tokens > 1 ? rope_copy_kernel<true> : rope_copy_kernel<false>)<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(src), static_cast<__nv_bfloat16*>(dst), cos_t, sin_t, T, S, H, Dh, rot_per_group,
       group_size);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -974,7 +974,7 @@ int mm_swiglu_fwd_rows(const void* gu, void* h, int64_t T, int F, const int* row
   } else {
     swiglu_fwd_kernel<false><<<blocks_for(total, 256), 128, 0, stream>>>(x, y, static_cast<uint32_t>(T), F, rows_dev);
   }
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_swiglu_fwd(const void* gu, void* h, int64_t T, int F, cudaStream_t stream) {
@@ -989,7 +989,7 @@ int mm_swiglu_bwd_rows(const void* gu, const void* dh, void* dgu, int64_t T, int
   swiglu_bwd_kernel<<<blocks_for(total, 128), 128, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh), static_cast<__nv_bfloat16*>(dgu),
       static_cast<uint32_t>(T), F, rows_dev);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_swiglu_bwd(const void* gu, const void* dh, void* dgu, int64_t T, int F, cudaStream_t stream) {
@@ -1004,7 +1004,7 @@ int mm_cross_entropy(void* logits, const int64_t* targets, float* loss, float* s
   auto* l = static_cast<__nv_bfloat16*>(logits);
   cross_entropy_kernel<<<static_cast<unsigned>(rows), CE_THREADS, 0, stream>>>(
       l, write_grad ? l : nullptr, targets, loss, stats_out, stats_in, V, ld, vocab_start, grad_scale);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -1015,7 +1015,7 @@ int mm_cross_entropy_to(const void* logits, void* grad, const int64_t* targets, 
   if (V % 8) return -2;
   cross_entropy_kernel<<<static_cast<unsigned>(rows), CE_THREADS, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(logits), static_cast<__nv_bfloat16*>(grad), targets, loss, nullptr, nullptr, V, V, 0, grad_scale);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -1031,7 +1031,7 @@ int mm_ce_combine(const int64_t* stats, int nranks, const int64_t* targets, floa
   for (int r = 0; r < nranks; ++r) a.stats[r] = reinterpret_cast<const float*>(stats[r]);
   a.nranks = nranks;
   ce_combine_kernel<<<blocks_for(rows, 256), 256, 0, stream>>>(a, targets, stats2, loss, rows);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -1043,7 +1043,7 @@ int mm_embedding_fwd(const void* table, const int64_t* ids, void* out, int64_t T
   embedding_fwd_kernel<<<blocks_for(total, 256), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(table), ids, static_cast<__nv_bfloat16*>(out), T, D,
       vocab_start, vocab_size, device_state() ? device_state()->status : nullptr);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_embedding_bwd(const void* dout, const int64_t* ids, float* grad, int64_t T, int D,
@@ -1054,7 +1054,7 @@ int mm_embedding_bwd(const void* dout, const int64_t* ids, float* grad, int64_t 
   embedding_bwd_kernel<<<blocks_for(total, 256), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(dout), ids, grad, T, D, vocab_start, vocab_size,
       device_state() ? device_state()->status : nullptr);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -1064,7 +1064,7 @@ int mm_add_bf16(const void* a, const void* b, void* out, int64_t n, cudaStream_t
   add_bf16_kernel<<<blocks_for(n / 8, 256), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(b),
       static_cast<__nv_bfloat16*>(out), n / 8);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_accumulate_f32_bf16(float* acc, const void* src, int64_t n, cudaStream_t stream) {
@@ -1072,7 +1072,7 @@ int mm_accumulate_f32_bf16(float* acc, const void* src, int64_t n, cudaStream_t 
   if (n == 0) return 0;
   accumulate_f32_bf16_kernel<<<blocks_for(n / 8, 256), 256, 0, stream>>>(
       acc, static_cast<const __nv_bfloat16*>(src), n / 8);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -1099,7 +1099,7 @@ static int launch_adamw(AdamwGroup g, bool ragged, float lr, float beta1, float 
   const float bc2 = 1.f - powf(beta2, static_cast<float>(step));
   auto kern = alone ? adamw_kernel<false> : adamw_kernel<true>;
   kern<<<blocks, 256, 0, stream>>>(g, lr, beta1, beta2, eps, wd, bc1, bc2, grad_scale, step_dev);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -1127,7 +1127,7 @@ int mm_sumsq_f32(const float* x, int64_t n, float* out, cudaStream_t stream) {
   DeviceState* ds = device_state();
   const int grid = ds ? ds->sm_count * 4 : 592;
   sumsq_f32_kernel<<<grid, 256, 0, stream>>>(x, n, out);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -1204,9 +1204,9 @@ extern "C" int mm_rmsnorm_bwd_noalloc(const void* x, const void* w, const void* 
   else if (D <= 4096) MM_RN_BWD_NA(128, 4);
   else MM_RN_BWD_NA(256, 4);
 #undef MM_RN_BWD_NA
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   // every block wrote its full row of partials above, so the reduction reads only fresh data
   colsum_partials_kernel<float, false, 8><<<(D + 31) / 32, 256, 0, stream>>>(scratch, dw_out, parts, D, accumulate_dw);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }

@@ -24,7 +24,7 @@ static int launch_plain(const CUtensorMap& tmA, const CUtensorMap& tmB, void* C,
   Hook hook{C, ldc, vec_ok, bn};
   GemmShape shape{M, N, K, nullptr, nullptr, bn};
   kern<<<grid, GEMM_THREADS, GEMM_SMEM_BYTES + Hook::kStageBytes, stream>>>(tmA, tmB, shape, hook, ds->status);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 

@@ -280,7 +280,7 @@ int mm_allgather_gemm_bf16(const int64_t* a_src, int nranks, int me, void* gathe
     }
     kern<<<grid, threads, GEMM_SMEM_BYTES, stream>>>(tmA, tmB, shape, hook, ds->status);
   }
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 

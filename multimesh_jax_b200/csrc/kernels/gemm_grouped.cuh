@@ -399,6 +399,7 @@ static int launch_grouped(Kernel kern, bool (&configured)[kMaxDevices], int64_t 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   MM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, args..., ds->status));
+  count_launches(1);
   return 0;
 }
 

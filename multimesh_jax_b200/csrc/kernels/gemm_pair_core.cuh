@@ -319,6 +319,7 @@ static int launch_pair_kernel(const CUtensorMap& tmA, const CUtensorMap& tmB, co
     fprintf(stderr, "[mm_kernels] paired GEMM launch failed: %s\n", cudaGetErrorString(cudaGetLastError()));
     return -1;
   }
+  count_launches(1);
   return 0;
 }
 

@@ -300,7 +300,7 @@ static int launch_linear_bwd(const CUtensorMap (&tm)[4], const LinearBwd& p, int
     configured[dev] = true;
   }
   kern<<<static_cast<unsigned>(ctas), GT_THREADS, smem, stream>>>(tm[0], tm[1], tm[2], tm[3], p, ds->status);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 template <int OUT_DW>
@@ -337,6 +337,7 @@ static int launch_tile(const CUtensorMap& tmA, const CUtensorMap& tmB, void* C, 
   cfg.attrs = attr;
   cfg.numAttrs = split > 1 ? 1 : 0;
   MM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, C, ldc, M, N, K, split, vec_ok, ds->status));
+  count_launches(1);
   return 0;
 }
 

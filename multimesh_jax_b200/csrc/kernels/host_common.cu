@@ -5,6 +5,8 @@
 
 namespace mm {
 
+std::atomic<int64_t> g_launches{0};
+
 static DeviceState g_states[kMaxDevices];
 static std::mutex g_mu;
 
@@ -133,6 +135,8 @@ void* mm_status_ptr() {
   mm::DeviceState* s = mm::device_state();
   return s ? s->status : nullptr;
 }
+
+int64_t mm_launch_count() { return mm::g_launches.load(std::memory_order_relaxed); }
 
 int mm_sm_count() {
   mm::DeviceState* s = mm::device_state();

@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 namespace mm {
 
 #define MM_CUDA_TRY(expr)                                                        \
@@ -17,6 +19,18 @@ namespace mm {
       return static_cast<int>(_e);                                               \
     }                                                                            \
   } while (0)
+
+// Behind the launch of `n` kernels: their error, or their count.
+#define MM_LAUNCHED(n)               \
+  do {                               \
+    MM_CUDA_TRY(cudaGetLastError()); \
+    ::mm::count_launches(n);         \
+  } while (0)
+
+// Kernels that this library has launched. An entry point takes one or several according to sizes and device, so they are
+// counted where they are launched.
+extern std::atomic<int64_t> g_launches;
+inline void count_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
 constexpr int kMaxDevices = 32;
 

@@ -232,7 +232,7 @@ int mm_moe_route_dispatch(const void* x, const void* wr, const void* other, int 
   const int threads = 256;
   const int blocks = (T * 32 + threads - 1) / threads;
   moe_route_dispatch_kernel<<<blocks, threads, 0, stream>>>(a, ds->status);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -254,7 +254,7 @@ int mm_moe_combine(const int64_t* buf, int nranks, const int* idx, const int* sl
   const int threads = 256;
   const int blocks = (T * 32 + threads - 1) / threads;
   moe_combine_kernel<<<blocks, threads, 0, stream>>>(a);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 

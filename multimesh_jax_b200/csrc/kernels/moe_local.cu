@@ -412,7 +412,7 @@ static int moe_group(const MoeSpace& w, const void* x, const void* wr, const voi
   ml_plan_kernel<<<E, 1024, 0, stream>>>(w.idx, T * k, E, w.plan, w.pos, w.row_of);
   ml_gather_kernel<<<w.cap, 128, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), w.xs, static_cast<const __nv_bfloat16*>(dy),
                                               dy ? w.ys : nullptr, w.row_of, w.plan, E, k, D);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(3);
   return 0;
 }
 
@@ -435,7 +435,7 @@ int mm_moe_route(const void* x, const void* wr, int* idx, float* gates, int T, i
   if (rc) return rc;
   ml_route_kernel<<<(T + ML_TOK - 1) / ML_TOK, 128, 0, stream>>>(static_cast<const __nv_bfloat16*>(x),
                                                                 static_cast<const __nv_bfloat16*>(wr), T, D, E, k, idx, gates);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -453,7 +453,7 @@ int mm_moe_fwd(const void* x, const void* wr, const void* wgu, const void* wdown
   if ((rc = grouped_rows(w.h, wdown, 0, w.rows, w.cap, E, D, F, w.plan, stream))) return rc;
   ml_combine_kernel<<<T, 128, 0, stream>>>(w.rows, w.idx, w.pos, w.gates, nullptr, nullptr, nullptr,
                                            static_cast<__nv_bfloat16*>(y), k, D);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(2);
   return 0;
 }
 
@@ -476,7 +476,7 @@ int mm_moe_bwd(const void* dy, const void* x, const void* wr, const void* wgu, c
   ml_dwr_kernel<<<dim3((D / 8 + 127) / 128, ML_DWR_SPLIT, E), 128, 0, stream>>>(w.xs, w.dl, w.row_of, w.plan, w.dwr_part, E, D);
   const int64_t n = static_cast<int64_t>(E) * D;
   ml_dwr_sum_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(w.dwr_part, static_cast<__nv_bfloat16*>(dwr), n);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(4);
   return 0;
 }
 

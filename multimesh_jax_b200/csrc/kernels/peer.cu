@@ -294,20 +294,20 @@ int mm_reshard_pull(const int64_t* chunks, int num_chunks, int elem_size, const 
   int grid = static_cast<int>(want < cap ? want : cap);
   if (grid < 1) grid = 1;
   reshard_pull_kernel<<<grid, 256, 0, stream>>>(args, ds->status);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
 int mm_set_flag(void* flag, int value, cudaStream_t stream) {
   set_flag_kernel<<<1, 1, 0, stream>>>(reinterpret_cast<int*>(flag), value);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_wait_flag(const void* flag, int value, cudaStream_t stream) {
   DeviceState* ds = device_state();
   if (!ds) return -1;
   wait_flag_kernel<<<1, 1, 0, stream>>>(reinterpret_cast<const int*>(flag), value, ds->status);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -327,7 +327,7 @@ int mm_peer_copy(void* dst, const void* src, int64_t bytes, cudaStream_t stream)
   const int cap = ds->sm_count * 8;
   const int grid = static_cast<int>(want < cap ? (want < 1 ? 1 : want) : cap);
   peer_copy_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), nvec);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -374,7 +374,7 @@ int mm_reduce_pull_chunked(const int64_t* srcs, int nsrc, void* out, int64_t chu
   const int cap = ds->sm_count * per_sm;
   const int grid = static_cast<int>(want < cap ? (want < 1 ? 1 : want) : cap);
   reduce_pull_kernel<<<grid, 256, 0, stream>>>(a);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -387,7 +387,7 @@ int mm_set_flags(const int64_t* flags, int n, int value, cudaStream_t stream) {
   f.n = n;
   for (int i = 0; i < n; ++i) f.flag[i] = reinterpret_cast<int*>(flags[i]);
   set_flags_kernel<<<1, 32, 0, stream>>>(f, value);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 // Holds the stream until up to eight local flags are >= `value`, for at most `limit_ms`
@@ -402,7 +402,7 @@ int mm_wait_flags(const int64_t* flags, int n, int value, int limit_ms, cudaStre
   for (int i = 0; i < n; ++i) f.flag[i] = reinterpret_cast<int*>(flags[i]);
   wait_flags_timeout_kernel<<<1, 32, 0, stream>>>(f, value, static_cast<unsigned long long>(limit_ms) * 1000000ull,
                                                   ds->status);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 

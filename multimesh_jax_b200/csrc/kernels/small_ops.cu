@@ -109,7 +109,7 @@ int mm_zero_row_tail(void* base, int64_t row_bytes, const int* count, int multip
   const int blocks = static_cast<int>((vecs + threads - 1) / threads);
   zero_row_tail_kernel<<<dim3(blocks, multiple), threads, 0, stream>>>(static_cast<uint4*>(base), vecs, count, multiple,
                                                                        capacity);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 
@@ -126,7 +126,7 @@ int mm_zero(void* dst, int64_t bytes, cudaStream_t stream) {
 int mm_f32_to_bf16(const float* src, void* dst, int64_t n, cudaStream_t stream) {
   if (n <= 0) return 0;
   f32_to_bf16_kernel<<<grid_for(n, 256, 4096), 256, 0, stream>>>(src, static_cast<__nv_bfloat16*>(dst), n);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 // dst(fp32) = src(bf16), or dst += src with accumulate != 0; any element count
@@ -134,24 +134,24 @@ int mm_bf16_to_f32(const void* src, float* dst, int64_t n, int accumulate, cudaS
   if (n <= 0) return 0;
   bf16_to_f32_kernel<<<grid_for(n, 256, 4096), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(src), dst, n,
                                                                  accumulate);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_accumulate_f32(float* acc, const float* src, int64_t n, cudaStream_t stream) {
   if (n <= 0) return 0;
   accumulate_f32_kernel<<<grid_for(n, 256, 4096), 256, 0, stream>>>(acc, src, n);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_fill_f32(float* dst, float value, int64_t n, cudaStream_t stream) {
   if (n <= 0) return 0;
   fill_f32_kernel<<<grid_for(n, 256, 4096), 256, 0, stream>>>(dst, value, n);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_sum_scale_f32(const float* src, int64_t n, float scale, float* out, cudaStream_t stream) {
   sum_scale_f32_kernel<<<1, 1024, 0, stream>>>(src, n, scale, out);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_scale_bf16(const void* x, const void* scalar, void* out, int64_t n, cudaStream_t stream) {
@@ -159,13 +159,13 @@ int mm_scale_bf16(const void* x, const void* scalar, void* out, int64_t n, cudaS
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return -2;
   scale_bf16_kernel<<<grid_for(n / 8 + 1, 256, 8192), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(scalar), static_cast<__nv_bfloat16*>(out), n);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 int mm_add_i64(const int64_t* src, int64_t delta, int64_t* dst, int64_t n, cudaStream_t stream) {
   if (n <= 0) return 0;
   add_i64_kernel<<<grid_for(n, 256, 65535), 256, 0, stream>>>(src, delta, dst, n);
-  MM_CUDA_TRY(cudaGetLastError());
+  MM_LAUNCHED(1);
   return 0;
 }
 

@@ -17,6 +17,7 @@ _P = c_void_p
 _SIGS = {
     "mm_read_status": (c_int, [c_int]),
     "mm_sm_count": (c_int, []),
+    "mm_launch_count": (c_int64, []),
     "mm_status_ptr": (c_void_p, []),
     "mm_set_peer_wait_ms": (c_int, [c_int]),
     "mm_gemm_bf16": (c_int, [_P, c_int, c_int64, _P, c_int, c_int64, _P, c_int, c_int64,
@@ -106,6 +107,11 @@ def load():
         fn.argtypes = args
     _LIB = lib
     return lib
+
+
+def launch_count() -> int:
+    """Kernels that the library has launched in this process (copies are not counted)."""
+    return _LIB.mm_launch_count() if _LIB is not None else 0
 
 
 def register(name: str, restype, argtypes) -> None:

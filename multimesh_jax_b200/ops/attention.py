@@ -70,7 +70,6 @@ def attention_fwd_packed(qkv: torch.Tensor, rep: int) -> Tuple[torch.Tensor, tor
     rc = _lib.load().mm_flash_attn_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), B, S, hkv, rep, D,
                                        K._stream())
     _lib.check(rc, "mm_flash_attn_fwd")
-    K._count()
     return out, lse
 
 
@@ -106,7 +105,6 @@ def attention_bwd_packed(dout: torch.Tensor, qkv: torch.Tensor, out: torch.Tenso
                                rope[1].data_ptr() if rope else None, B, S, hkv, rep, D,
                                K._stream())
     _lib.check(rc, "mm_flash_attn_bwd")
-    K._count(1 if S <= 128 else 3)      # one block: the kernel needs none ahead or behind
     return dqkv
 
 

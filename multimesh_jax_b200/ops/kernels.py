@@ -18,10 +18,14 @@ from . import _lib
 
 bf16 = torch.bfloat16
 
-# Number of kernel launches issued through this module (for benchmarks), and the number of
-# calls that went to a vendor-library kernel instead of one of ours.
-launch_count = 0
+# The number of calls that went to a vendor-library kernel instead of one of ours.
 library_call_count = 0
+
+
+def __getattr__(name: str):
+    if name == "launch_count":      # kernels of the in-tree library that this process has launched
+        return _lib.launch_count()
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def count_library_call(n: int = 1) -> None:
@@ -32,11 +36,6 @@ def count_library_call(n: int = 1) -> None:
 def _stream() -> int:
     # the handle without a Stream object around it: every eager operator asks for it
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
-
-
-def _count(n: int = 1) -> None:
-    global launch_count
-    launch_count += n
 
 
 def read_status(clear: bool = True) -> int:
@@ -166,7 +165,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
                                        m_dev.data_ptr() if m_dev is not None else None,
                                        k_dev.data_ptr() if k_dev is not None else None, _stream())
         _lib.check(rc, "mm_gemm_pair_dyn_bf16")
-        _count()
         return out
     args = (a.data_ptr(), int(a_mn), a.stride(0), b.data_ptr(), int(b_mn), b.stride(0), out.data_ptr(), mode, out.stride(0),
             M, N, K)
@@ -175,7 +173,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     else:
         fn = lib.mm_gemm_pair_bf16 if pair else lib.mm_gemm_bf16
         _lib.check(fn(*args, _stream()), "mm_gemm_pair_bf16" if pair else "mm_gemm_bf16")
-    _count()
     return out
 
 
@@ -216,7 +213,6 @@ def zero_row_tail(x: torch.Tensor, rows: torch.Tensor, multiple: int = 64) -> No
     rc = _lib.load().mm_zero_row_tail(x.data_ptr(), x.shape[1] * x.element_size(), rows.data_ptr(), multiple, x.shape[0],
                                       _stream())
     _lib.check(rc, "mm_zero_row_tail")
-    _count()
 
 
 # ------------------------------------------------------------------ RMSNorm
@@ -234,7 +230,6 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float) -> Tuple[torch.Ten
     rc = _lib.load().mm_rmsnorm_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), rows, D,
                                     eps, _stream())
     _lib.check(rc, "mm_rmsnorm_fwd")
-    _count()
     return y, rstd
 
 
@@ -252,7 +247,6 @@ def add_rmsnorm_fwd(x: torch.Tensor, delta: torch.Tensor, w: torch.Tensor,
     rc = _lib.load().mm_add_rmsnorm_fwd(x.data_ptr(), delta.data_ptr(), xn.data_ptr(), w.data_ptr(), y.data_ptr(),
                                         rstd.data_ptr(), rows, D, eps, _stream())
     _lib.check(rc, "mm_add_rmsnorm_fwd")
-    _count()
     return xn, y, rstd
 
 
@@ -305,7 +299,6 @@ def rmsnorm_bwd(x: torch.Tensor, w: torch.Tensor, dy: torch.Tensor, rstd: torch.
                             dw_out.data_ptr(), scratch.data_ptr(), rows, D, int(accumulate_dw),
                             int(dx_inout is not None), _stream())
     _lib.check(rc, "mm_rmsnorm_bwd")
-    _count(2)
     return dx, dw_out
 
 
@@ -341,7 +334,6 @@ def rope_(qk: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, backward: bool
     rc = _lib.load().mm_rope(qk.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, S, n_rot, Dh, qk.stride(0),
                              int(backward), rot_per_group, group_size, _stream())
     _lib.check(rc, "mm_rope")
-    _count()
     return qk
 
 
@@ -355,7 +347,6 @@ def rope(qk: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, rot_per_group: 
     rc = _lib.load().mm_rope_copy(qk.data_ptr(), out.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, cos.shape[0], H, Dh,
                                   rot_per_group, group_size, _stream())
     _lib.check(rc, "mm_rope_copy")
-    _count()
     return out
 
 
@@ -372,7 +363,6 @@ def swiglu_fwd(gu: torch.Tensor, rows: Optional[torch.Tensor] = None) -> torch.T
     rc = _lib.load().mm_swiglu_fwd_rows(gu.data_ptr(), h.data_ptr(), T, F, rows.data_ptr() if rows is not None else None,
                                         _stream())
     _lib.check(rc, "mm_swiglu_fwd")
-    _count()
     return h
 
 
@@ -389,7 +379,6 @@ def swiglu_bwd(gu: torch.Tensor, dh: torch.Tensor, rows: Optional[torch.Tensor] 
     rc = _lib.load().mm_swiglu_bwd_rows(gu.data_ptr(), dh.contiguous().data_ptr(), dgu.data_ptr(), T, F,
                                         rows.data_ptr() if rows is not None else None, _stream())
     _lib.check(rc, "mm_swiglu_bwd")
-    _count()
     return dgu
 
 
@@ -415,7 +404,6 @@ def cross_entropy_fwd_bwd(logits: torch.Tensor, targets: torch.Tensor, grad_scal
     rc = _lib.load().mm_cross_entropy(logits.data_ptr(), targets.data_ptr(), loss.data_ptr(), None, None,
                                       rows, V, logits.stride(0), 0, grad_scale, int(write_grad), _stream())
     _lib.check(rc, "mm_cross_entropy")
-    _count()
     return loss
 
 
@@ -429,7 +417,6 @@ def cross_entropy_to(logits: torch.Tensor, targets: torch.Tensor, grad_scale: fl
         rc = _lib.load().mm_cross_entropy_to(logits.data_ptr(), grad.data_ptr(), targets.data_ptr(), loss.data_ptr(), rows, V,
                                              grad_scale, _stream())
         _lib.check(rc, "mm_cross_entropy_to")
-        _count()
         return loss, grad
     grad = logits.clone()
     return cross_entropy_fwd_bwd(grad, targets, grad_scale), grad
@@ -451,7 +438,6 @@ def cross_entropy_stats(logits: torch.Tensor, targets: torch.Tensor, vocab_start
     rc = _lib.load().mm_cross_entropy(logits.data_ptr(), targets.data_ptr(), None, stats.data_ptr(), None, rows, V,
                                       logits.stride(0), vocab_start, 0.0, 0, _stream())
     _lib.check(rc, "mm_cross_entropy")
-    _count()
     return stats
 
 
@@ -475,7 +461,6 @@ def cross_entropy_combine(all_stats, targets: torch.Tensor, stat_ptrs=None):
     rc = _lib.load().mm_ce_combine(arr, len(stat_ptrs), targets.data_ptr(), stats2.data_ptr(), loss.data_ptr(), rows,
                                    _stream())
     _lib.check(rc, "mm_ce_combine")
-    _count()
     return stats2, loss
 
 
@@ -496,7 +481,6 @@ def cross_entropy_apply(logits: torch.Tensor, targets: torch.Tensor, stats2: tor
     rc = _lib.load().mm_cross_entropy(logits.data_ptr(), targets.data_ptr(), None, None, stats2.data_ptr(), rows, V,
                                       logits.stride(0), vocab_start, grad_scale, 1, _stream())
     _lib.check(rc, "mm_cross_entropy")
-    _count()
 
 
 # ---------------------------------------------------------------- embedding
@@ -512,7 +496,6 @@ def embedding_fwd(table: torch.Tensor, ids: torch.Tensor, vocab_start: int = 0) 
     rc = _lib.load().mm_embedding_fwd(table.data_ptr(), flat.data_ptr(), out.data_ptr(), flat.numel(), D,
                                       vocab_start, V, _stream())
     _lib.check(rc, "mm_embedding_fwd")
-    _count()
     return out
 
 
@@ -528,7 +511,6 @@ def embedding_bwd(dout: torch.Tensor, ids: torch.Tensor, grad: torch.Tensor, voc
     rc = _lib.load().mm_embedding_bwd(dout.contiguous().data_ptr(), flat.data_ptr(), grad.data_ptr(),
                                       flat.numel(), D, vocab_start, V, _stream())
     _lib.check(rc, "mm_embedding_bwd")
-    _count()
     return grad
 
 
@@ -539,7 +521,6 @@ def add_(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
         return a.add_(b)
     rc = _lib.load().mm_add_bf16(a.data_ptr(), b.data_ptr(), a.data_ptr(), a.numel(), _stream())
     _lib.check(rc, "mm_add_bf16")
-    _count()
     return a
 
 
@@ -549,7 +530,6 @@ def add(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     out = torch.empty_like(a)
     rc = _lib.load().mm_add_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), a.numel(), _stream())
     _lib.check(rc, "mm_add_bf16")
-    _count()
     return out
 
 
@@ -559,7 +539,6 @@ def accumulate_(acc: torch.Tensor, src: torch.Tensor) -> torch.Tensor:
         return acc.add_(src.to(acc.dtype))
     rc = _lib.load().mm_accumulate_f32_bf16(acc.data_ptr(), src.contiguous().data_ptr(), acc.numel(), _stream())
     _lib.check(rc, "mm_accumulate_f32_bf16")
-    _count()
     return acc
 
 
@@ -588,7 +567,6 @@ def adamw_step_(master: torch.Tensor, param: torch.Tensor, m: torch.Tensor, v: t
                               1 if step_t is not None else int(step), grad_scale,
                               step_t.data_ptr() if step_t is not None else None, _stream())
     _lib.check(rc, "mm_adamw")
-    _count()
 
 
 def sumsq(x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
@@ -598,7 +576,6 @@ def sumsq(x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         return out
     rc = _lib.load().mm_sumsq_f32(x.data_ptr(), x.numel(), out.data_ptr(), _stream())
     _lib.check(rc, "mm_sumsq_f32")
-    _count()
     return out
 
 

@@ -148,7 +148,6 @@ def _route_as_grouped(x2: torch.Tensor, wr: torch.Tensor, top_k: int) -> Tuple[t
     rc = _lib.load().mm_moe_route(x2.data_ptr(), wr.data_ptr(), idx.data_ptr(), gates.data_ptr(), T, D, wr.shape[0], top_k,
                                   K._stream())
     _lib.check(rc, "mm_moe_route")
-    K._count()
     return idx.long(), gates
 
 
@@ -164,7 +163,6 @@ def moe_ffn_impl(x, wr, wgu, wdown, top_k: int):
         rc = _lib.load().mm_moe_fwd(x2.data_ptr(), wr.data_ptr(), wgu.data_ptr(), wdown.data_ptr(), y.data_ptr(),
                                     ws.data_ptr(), x2.shape[0], D, F, E, top_k, K._stream())
         _lib.check(rc, "mm_moe_fwd")
-        K._count(7)
         return y.view(x.shape)
     topi, gates = _route_as_grouped(x2, wr, top_k) if need is not None else route(x2, wr, top_k)[1:]
     y = torch.zeros(x2.shape, dtype=torch.float32, device=x.device)
@@ -194,7 +192,6 @@ def moe_ffn_bwd_impl(dy, x, wr, wgu, wdown, top_k: int):
                                     dx.data_ptr(), dwr.data_ptr(), dwgu.data_ptr(), dwdown.data_ptr(), ws.data_ptr(),
                                     x2.shape[0], D, F, E, top_k, K._stream())
         _lib.check(rc, "mm_moe_bwd")
-        K._count(12)
         return dx.view(x.shape), dwr, dwgu, dwdown
     topi, gates = _route_as_grouped(x2, wr, top_k) if need is not None else route(x2, wr, top_k)[1:]
     dx = torch.zeros(x2.shape, dtype=torch.float32, device=x.device)

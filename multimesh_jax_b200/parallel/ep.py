@@ -95,7 +95,6 @@ class PeerMoE:
                                             self._ptrs(self.counter), self.n, idx.data_ptr(), gates.data_ptr(),
                                             slot.data_ptr(), _stream())
         _lib.check(rc, "mm_moe_route_dispatch")
-        K._count()
         return idx, gates, slot
 
     def _counts(self) -> List[int]:
@@ -124,7 +123,6 @@ class PeerMoE:
                                      y.data_ptr() if y is not None else None, T, self.D, self.k, self.E_l, self.capacity,
                                      _stream())
         _lib.check(rc, "mm_moe_combine")
-        K._count()
 
     # ------------------------------------------------------------------
     def forward(self, x2: torch.Tensor, wr: torch.Tensor, wgu: torch.Tensor, wdown: torch.Tensor, top_k: int):

@@ -78,7 +78,6 @@ class PeerGroupComm:
         srcs = (c_int64 * g)(*[s_in.ptr(r) + me * share for r in self.ranks])
         rc = K_lib.mm_reduce_pull(srcs, g, s_red.ptr(a.rank) + me * share, share, x.element_size(), scale, stream)
         _lib.check(rc, "mm_reduce_pull")
-        K._count()
         self.barrier()                                    # every member's share is reduced
         if out is None:
             out = torch.empty_like(x)                     # else in place: x was staged above, its buffer is free
@@ -86,7 +85,6 @@ class PeerGroupComm:
             one = (c_int64 * 1)(s_red.ptr(r) + i * share)
             rc = K_lib.mm_reduce_pull(one, 1, out.data_ptr() + i * share, share, x.element_size(), 1.0, stream)
             _lib.check(rc, "mm_reduce_pull")
-            K._count()
         self.barrier()                                    # staging tiles may be overwritten again
         self.calls += 1
         return out
@@ -144,7 +142,6 @@ class PeerGroupComm:
         rc = a.lib.mm_reduce_pull_chunked(srcs, g, out.data_ptr(), chunk, outer, stride, x.element_size(), scale,
                                           torch.cuda.current_stream().cuda_stream)
         _lib.check(rc, "mm_reduce_pull_chunked")
-        K._count()
         self.barrier()                                # staging tiles may be overwritten again
         self.calls += 1
         return out

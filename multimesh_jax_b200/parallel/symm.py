@@ -271,7 +271,6 @@ def reshard_pull(records: List[List[int]], elem_size: int, arena: SymmetricArena
                              len(done_flags), done_value, arena.counter_ptr(counter) if done_flags else None, max_ctas,
                              torch.cuda.current_stream().cuda_stream)
     _lib.check(rc, "mm_reshard_pull")
-    K._count()
 
 
 def set_flags(arena: SymmetricArena, ptrs: Sequence[int], value: int) -> None:
@@ -280,7 +279,6 @@ def set_flags(arena: SymmetricArena, ptrs: Sequence[int], value: int) -> None:
         part = list(ptrs[i:i + 8])
         arr = (c_int64 * len(part))(*part)
         _lib.check(arena.lib.mm_set_flags(arr, len(part), value, torch.cuda.current_stream().cuda_stream), "mm_set_flags")
-        K._count()
 
 
 def wait_flags(arena: SymmetricArena, ptrs: Sequence[int], value: int, limit_ms: int = 30000) -> None:
@@ -291,4 +289,3 @@ def wait_flags(arena: SymmetricArena, ptrs: Sequence[int], value: int, limit_ms:
         arr = (c_int64 * len(part))(*part)
         _lib.check(arena.lib.mm_wait_flags(arr, len(part), value, limit_ms, torch.cuda.current_stream().cuda_stream),
                    "mm_wait_flags")
-        K._count()

@@ -75,7 +75,6 @@ class FusedLinearAllReduce:
                                              flag_local, flag_peer, npeers, bs.epoch,
                                              torch.cuda.current_stream().cuda_stream)
         _lib.check(rc, "mm_gemm_allreduce_bf16")
-        K._count()
         self.calls += 1
         return out
 
@@ -152,7 +151,6 @@ class FusedLinearReduceScatter:
                                                  flag_local, flag_peer, g, me, chunk_rows, bs.epoch,
                                                  torch.cuda.current_stream().cuda_stream)
         _lib.check(rc, "mm_gemm_reducescatter_bf16")
-        K._count()
         self.calls += 1
         return out
 
@@ -240,6 +238,5 @@ class FusedAllGatherLinear:
                                              Ms // outer, shard_ready, self.epoch, a_shard.data_ptr(),
                                              torch.cuda.current_stream().cuda_stream)
         _lib.check(rc, "mm_allgather_gemm_bf16")
-        K._count()
         self.calls += 1
         return out, gathered

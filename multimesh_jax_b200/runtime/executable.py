@@ -970,7 +970,6 @@ class Executable:
             bases.extend(t.data_ptr() for t in ext_tiles)
             bases.extend(b_.data_ptr() for b_ in blocks[1:])
             native.kernel.launch(bases, scalars, K._stream())
-            K._count(native.num_calls)
             self.native_launches += 1
             typed_blocks: Dict[Tuple[int, torch.dtype], torch.Tensor] = {}
             for pos, (spec, s) in enumerate(zip(out_specs, out_ids)):
