@@ -384,7 +384,7 @@ struct GemmChoice {
   int bn, split, cols;
   bool pair;
 };
-static GemmChoice gemm_choose(int out_mode, int M, int N, int K, int pair_min_m, int sm) {
+static GemmChoice gemm_choose(int out_mode, int M, int N, int K, bool b_mn, int64_t lda, int64_t ldb, int pair_min_m, int sm) {
   const double kb = (K + GT_BK - 1) / GT_BK;
   auto blocks = [&](int bm, int bn) { return static_cast<double>((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
   auto rounds = [](double ctas, int at_once) { return ceil(ctas / at_once); };
@@ -417,12 +417,19 @@ static GemmChoice gemm_choose(int out_mode, int M, int N, int K, int pair_min_m,
       if (t < best) { best = t; bn = n; split = s; }
     }
   }
+  // narrower tiles: see mm_gemm_auto_bf16
   int cols = bn ? 0 : 256;      // of a persistent tile
   double narrow = 0.95 * best;
-  for (int n = 128; n < 256; n += 16)
-    if (single_time(n) < narrow) { narrow = single_time(n); pair = false; cols = n; }
-  for (int n = 128; pairs && n < 256; n += 32)
-    if (pair_time(n) < narrow) { narrow = pair_time(n); pair = true; cols = n; }
+  if (bn || pair) {
+    const bool sectors = lda % 16 == 0 && ldb % 16 == 0;
+    const bool one_round = bn == 64 && blocks(128, 64) * split <= 2 * sm;
+    if (pairs && narrow > 5.3 && (!b_mn || sectors) && !one_round && !(acc && kb < (bn ? 8 : 4)))
+      for (int n = 128; n < 256; n += 32)
+        if (pair_time(n) < narrow) { narrow = pair_time(n); pair = true; cols = n; }
+  } else if (!b_mn && narrow > 6.0) {
+    for (int n = 128; n < 256; n += 16)
+      if (single_time(n) < narrow) { narrow = single_time(n); cols = n; }
+  }
   return GemmChoice{bn, split, cols, pair};
 }
 
@@ -455,6 +462,13 @@ int mm_gemm_tile_bf16(const void* A, int a_mn, int64_t lda, const void* B, int b
   return -2;
 }
 
+static int run_choice(const mm::GemmChoice& c, const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C,
+                      int out_mode, int64_t ldc, int M, int N, int K, cudaStream_t stream) {
+  if (!c.cols) return mm_gemm_tile_bf16(A, a_mn, lda, B, b_mn, ldb, C, out_mode, ldc, M, N, K, c.bn, c.split, stream);
+  return c.pair ? mm_gemm_pair_cols_bf16(A, a_mn, lda, B, b_mn, ldb, C, out_mode, ldc, M, N, K, c.cols, stream)
+                : mm_gemm_cols_bf16(A, a_mn, lda, B, b_mn, ldb, C, out_mode, ldc, M, N, K, c.cols, stream);
+}
+
 // Same contract as mm_gemm_bf16; picks the kernel by an estimate of its time in microseconds. Fitted on one
 // B200 to cold operands of 64..8192 rows, 256..28672 columns and K 256..28672, where the choice was within
 // 8 % of the best of all kernels; both sides where two of them meet (bf16, us):
@@ -481,7 +495,14 @@ int mm_gemm_tile_bf16(const void* A, int a_mn, int64_t lda, const void* B, int b
 //    2600 2048 2048   32.8  27.5 (pair, 160)    2048 12288 4096  137.2 123.7 (pair, 224)     600 4096 2048  22.5 20.5 (pair, 192)
 //    1024 2816 1500   26.6  23.1 (fp32 accumulation, pair, 160)   5632 1024 1500  38.9  34.8 (the same, 192)
 //     333 28672 4096  94.2  90.1 (single, 208; bound by what L2 gives out)
-// Of 182 problems of model layers 33 change, 26 of them by 3..16 %, four lose 4..12 % (long contractions).
+// Only the columns of the kernel that won on full tiles are narrowed (pairs also take over from small tiles that are more
+// than the chip holds at once), and not where the narrow tile reads as much as the full one or where that costs most:
+//   MN-major B comes in slabs of 64 columns, so that single tiles of 144 read 192: 612 4096 7416 52.9 -> 68.7 on them
+//   rows that do not start on the 32 bytes of a sector (MN-major B, whose tiles start anywhere): 1496 4096 3200, rows of
+//     1496, 43.8 -> 49.2; 2743 1024 25128 157 -> 181
+//   sums into the result over a few K blocks, where reading the result is most of the time: 5120 1024 128 20.8 -> 23.4
+// Of 501 problems whose tile changes (model layers and odd sizes up to 8192 rows) the mean gain is 1.12 and five are slower
+// by more than 2 %; of 40 whose tile stays two are, which is how far two runs of one kernel differ.
 // pair_min_m: CTA pairs from this many rows on; 0: never.
 int mm_gemm_auto_bf16(const void* A, int a_mn, int64_t lda, const void* B, int b_mn, int64_t ldb, void* C, int out_mode,
                       int64_t ldc, int M, int N, int K, int pair_min_m, cudaStream_t stream) {
@@ -489,10 +510,8 @@ int mm_gemm_auto_bf16(const void* A, int a_mn, int64_t lda, const void* B, int b
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   DeviceState* ds = device_state();
   if (!ds) return -1;
-  const GemmChoice c = gemm_choose(out_mode, M, N, K, pair_min_m, ds->sm_count);
-  if (!c.cols) return mm_gemm_tile_bf16(A, a_mn, lda, B, b_mn, ldb, C, out_mode, ldc, M, N, K, c.bn, c.split, stream);
-  return c.pair ? mm_gemm_pair_cols_bf16(A, a_mn, lda, B, b_mn, ldb, C, out_mode, ldc, M, N, K, c.cols, stream)
-                : mm_gemm_cols_bf16(A, a_mn, lda, B, b_mn, ldb, C, out_mode, ldc, M, N, K, c.cols, stream);
+  return run_choice(gemm_choose(out_mode, M, N, K, b_mn != 0, lda, ldb, pair_min_m, ds->sm_count), A, a_mn, lda, B, b_mn, ldb, C,
+                    out_mode, ldc, M, N, K, stream);
 }
 
 // dx[T, K] = dy[T, N] w[N, K] (bf16) and dw[N, K] (+)= dy^T x[T, K] (dw_mode: an out_mode of mm_gemm_bf16); everything
@@ -504,13 +523,14 @@ int mm_linear_bwd_bf16(const void* dy, const void* w, const void* x, void* dx, v
   if (T <= 0 || N <= 0 || K <= 0) return 0;
   DeviceState* ds = device_state();
   if (!ds) return -1;
-  const GemmChoice a = gemm_choose(OUT_BF16, T, K, N, pair_min_m, ds->sm_count), b = gemm_choose(dw_mode, N, K, T, pair_min_m, ds->sm_count);
+  const GemmChoice a = gemm_choose(OUT_BF16, T, K, N, true, N, K, pair_min_m, ds->sm_count);
+  const GemmChoice b = gemm_choose(dw_mode, N, K, T, true, N, K, pair_min_m, ds->sm_count);
   auto ctas = [](int rows, int cols, int bn) { return static_cast<int64_t>((rows + GT_BM - 1) / GT_BM) * ((cols + bn - 1) / bn); };
   const bool aligned = N % 8 == 0 && K % 8 == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
   if (!aligned || dw_mode == OUT_BF16_ACC || a.cols || b.cols || a.split > 1 || b.split > 1 ||
       ctas(T, K, a.bn) + ctas(N, K, b.bn) > ds->sm_count) {
-    const int rc = mm_gemm_auto_bf16(dy, 0, N, w, 1, K, dx, OUT_BF16, K, T, K, N, pair_min_m, stream);
-    return rc ? rc : mm_gemm_auto_bf16(dy, 1, N, x, 1, K, dw, dw_mode, K, N, K, T, pair_min_m, stream);
+    const int rc = run_choice(a, dy, 0, N, w, 1, K, dx, OUT_BF16, K, T, K, N, stream);
+    return rc ? rc : run_choice(b, dy, 1, N, x, 1, K, dw, dw_mode, K, N, K, T, stream);
   }
   CUtensorMap tm[4];
   int rc = encode_tmap_2d_bf16(&tm[0], dy, N, T, static_cast<uint64_t>(N) * 2, GT_BK, GT_BM);
