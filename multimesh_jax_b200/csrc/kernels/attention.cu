@@ -83,7 +83,12 @@ struct BlockOrder {
   int heads, group, nblk;   // heads in all, heads of a group, blocks of a head
   // `rank`: 0 for the longest block of its head
   __device__ __forceinline__ void at(int t, int& head, int& rank) const {
-    const int gi = t / (group * nblk);
+    if (nblk == 1) {      // every head one block: a short call feels two divisions
+      head = t;
+      rank = 0;
+      return;
+    }
+    const int gi = t < group * nblk ? 0 : t / (group * nblk);
     const int within = t - gi * (group * nblk);
     const int n = min(group, heads - gi * group);
     rank = within / n;
@@ -974,9 +979,11 @@ static int packed_map(CUtensorMap* out, const void* base, int B, int S, int H, i
 
 // CTAs of a cluster that share the query heads of one key block. More of them shorten the longest block (all heads
 // against the first keys) but each repeats the block's fixed part and the cluster adds its gradients at the end. In steps
-// of 128 x 128 (3.4 us): 2 for a block's start and end, 1.5 more for a cluster and 0.3 for each of its CTAs (fitted to
-// 150 measured shapes x splits, S 64 to 8192, 1 to 128 KV heads, rep 2 to 8; the choice is 0.5 % from the best of them
-// on average, 20 % at most). The blocks of one round last as long as the longest, more than a round as long as the
+// of 128 x 128 (3.4 us in the mean of the fitted shapes; 2.7 us on B1 S8192 32/8 heads): 2 for a block's start and end,
+// 1.5 more for a cluster and 0.3 for each of its CTAs (fitted to 150 measured shapes x splits, S 64 to 8192, 1 to 128 KV
+// heads, rep 2 to 8; the choice is 0.5 % from the best of them on average, 20 % at most). Where a sequence is one block its
+// steps take 4.0 us, with their row statistics, and a cluster costs 1.4 of them whatever its size: B8 S64 32/8 heads 23.1
+// us unsplit, 21.5 over two CTAs (21.2 in steps of 64 rows, before), B8 S128 32/8 26.5 | 24.1, B16 S64 32/4 39.2 | 29.8. The blocks of one round last as long as the longest, more than a round as long as the
 // chip's share of all of them and one of the shortest, which ends last. Splitting whenever the longest block exceeded
 // the chip's share of the steps alone was 15 % from the best: B16 S128 32/8 heads 50 us against 31 unsplit, B2 S1000
 // 32/8 heads 108 against 72 over two CTAs.
@@ -984,7 +991,7 @@ static int bwd_split(int64_t kv_heads, int rep, int nqb, int sms) {
   int best = 1;
   double best_time = 0;
   for (int s = 1; s <= 8 && rep % s == 0; s *= 2) {
-    const double fixed = s == 1 ? 2.0 : 3.5 + 0.3 * s;
+    const double fixed = s == 1 ? 2.0 : nqb == 1 ? 3.4 : 3.5 + 0.3 * s;
     const double blocks = static_cast<double>(kv_heads) * nqb * s, steps = static_cast<double>(kv_heads) * rep * nqb * (nqb + 1) / 2;
     double time = static_cast<double>(nqb) * rep / s + fixed;
     if (blocks > sms) time = std::max(time, (steps + fixed * blocks) / sms + static_cast<double>(rep) / s + fixed);
