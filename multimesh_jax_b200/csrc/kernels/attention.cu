@@ -33,8 +33,8 @@
 //   elected issue with ready descriptors (ptx.cuh)      B1 S8192 32 / 8 heads  3.04 -> 2.85, B4 H16 S1000 0.249 -> 0.233
 //   forward: exponentials ahead of the wait for the previous product, maximum and sum as four chains each, the
 //     scale inside the exponent's multiply-add          B1 S8192 32 / 8 heads  2.83 -> 2.77
-//   forward: P through TMEM, not shared memory: of the 1,024 cycles that a step's shared-memory traffic takes
-//     (reads of S 384 and P V 256, K and V tiles 256, P 128) 256 go, against 512 of the tensor cores
+//   forward: P through TMEM, not shared memory: at 128 bytes a cycle a step's shared-memory traffic is 1,024 cycles
+//     (reads of S 384 and P V 256, K and V tiles 256, P 128), of which 256 go, against 512 of the tensor cores
 //                                                       B1 S8192 32 / 8 heads  0.502 -> 0.460, B4 S2048 32 heads 0.171 -> 0.160
 //   backward: steps of 128 query rows (N = 64 instructions take as long as N = 128), P^T as an operand in TMEM, dQ by
 //     bulk reductions, a KV group's query heads over a cluster where a block would outlast the rest
@@ -42,9 +42,11 @@
 //                 B3 S500 8 / 2 heads    0.080 -> 0.045  B1 S1500 6 / 2 heads 0.139 -> 0.106  B2 S128 2 heads    0.031 -> 0.025
 //     dK and dV in one kernel and dQ in another (seven products instead of five, no sums in memory): 1.52 ms and
 //     0.595 ms on the two largest; better only below a dozen blocks
-// What bounds it: backward, shared memory: a step's products read 2,304 cycles of it (S, dP, dK, dQ 512 each, dV 256), the Q
-// and dO tiles write 512, dS 256, dQ passes through twice (1,024) and the row statistics take 256, together about the
-// 4,200 cycles that a step takes against 2,560 of the tensor cores; forward, shared memory and the exponentials.
+// What bounds it, by counters of B1 S8192 32 / 8 heads: no unit alone. Backward: a step of 128 x 128 is 4,200 cycles, the
+// tensor pipe active in 58 % of them; loads and stores of shared memory take 45 % (a third of it bank conflicts), its
+// banks are read at 33 % and written at 15 % of their peak, memory is at 10 %. One block per SM has one chain in flight:
+// scores, probabilities, dP, dS, dQ, whose columns the next dP waits for. Forward, two blocks per SM: tensor pipe 60 %,
+// banks 30 and 16 %, memory 4 %; beside it the exponentials, one per score on the special-function unit.
 #include <math.h>
 
 #include <algorithm>
