@@ -158,6 +158,21 @@ def test_norm_gradient_of_small_and_large_rows(rows, D, accumulate, add):
     assert ((dw.double() - dw_want).norm() <= 4 * rows ** 0.5 * 2.0 ** -24 * dw_want.norm().clamp_min(1.0))
 
 
+# the same sums rounded to the weight's type, and rounded before they are added: one cluster of each width, two launches
+@pytest.mark.parametrize("rows,D", [(3, 248), (257, 256), (129, 264), (257, 504), (256, 512), (257, 512), (600, 1032)])
+def test_norm_gradient_is_rounded_as_the_weight_is(rows, D):
+    x, dy, w, rstd = _rand(rows, D), _rand(rows, D), _rand(D), torch.rand(rows, device="cuda") + 0.5
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    scratch, dx = torch.empty(lib.mm_rmsnorm_bwd_parts(rows) * D, device="cuda"), torch.empty_like(x)
+    ins = [t.data_ptr() for t in (x, w, dy, rstd, dx)]
+    full, half, acc = torch.empty(D, device="cuda"), torch.empty(D, device="cuda").bfloat16(), torch.randn(D, device="cuda")
+    want = acc.clone()
+    assert lib.mm_rmsnorm_bwd(*ins, full.data_ptr(), scratch.data_ptr(), rows, D, 0, 0, stream) == 0
+    assert lib.mm_rmsnorm_bwd_bf16(*ins, half.data_ptr(), scratch.data_ptr(), rows, D, 0, stream) == 0
+    assert lib.mm_rmsnorm_bwd_acc(*ins, acc.data_ptr(), scratch.data_ptr(), rows, D, 1, 0, stream) == 0
+    assert torch.equal(half, full.bfloat16()) and torch.equal(acc, want + half.float())
+
+
 @pytest.mark.parametrize("rows,V", [(1, 8), (300, 2056), (70, 32000)])
 def test_loss_gradient_into_another_buffer(rows, V):
     logits, targets = _rand(rows, V), torch.randint(0, V, (rows,), device="cuda")
