@@ -625,7 +625,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1)
         umma_commit(ds_free);
       }
     }
-    __syncwarp();
   } else if (warp >= 12) {
     // dQ leaves TMEM as soon as it is complete (the next step's dP^T waits for its columns) and is added to memory by
     // bulk reductions, half a tile at a time through shared memory. As instructions (red.global.add.v4, straight from the
